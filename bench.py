@@ -366,7 +366,7 @@ def run_ours(args):
         phase_ms[1] += ph["adjoint_ms"]
         run_ms.append(tm["run_ms"])
         step_ms.append(tm["step_ms"])
-        launches += tm["step_launches"] + 2 + len(jobs)   # step kernels + source seeding + residuals
+        launches += plan.launches() + 2 + len(jobs)   # step kernels + source seeding + residuals
     barrier_sync(world)
     wall = time.perf_counter() - t0
     clocks = sampler.stop()

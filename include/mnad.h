@@ -63,7 +63,12 @@ enum { MNAD_SNAP_F32 = 0, MNAD_SNAP_BF16 = 1, MNAD_SNAP_F16 = 2 };
 enum { MNAD_PAIR_REFERENCE = 0, MNAD_PAIR_ALIGNED = 1 };
 
 /* Step kernel choice.  AUTO picks per launch group (propagations of one grid
- * size advancing together): the persistent TMA kernel once a launch has about
+ * size advancing together).  Where the state of one propagation fits the SMs'
+ * shared memory (up to about 0.7M points) it is RESIDENT: the on-chip kernel,
+ * which runs all steps of a propagation in one launch; its outputs are bitwise
+ * those of the kernel AUTO would take without it.  RESIDENT is reported by
+ * mnad_plan_kernels and cannot be set.  Otherwise: the persistent TMA kernel
+ * once a launch has about
  * 2.25 of its 64 x 16 tiles per resident CTA (0.7M point-updates on a 152-SM
  * GB300) -- on 64 x 8 tiles (TMA_NARROW) where the CPML strips hold under
  * 15 % of the grid's points, on 64 x 16 tiles otherwise -- and the
@@ -88,7 +93,8 @@ enum {
     MNAD_KERNEL_TMA = 2,
     MNAD_KERNEL_TUNE = 3,
     MNAD_KERNEL_TMA2 = 4,
-    MNAD_KERNEL_TMA_NARROW = 5
+    MNAD_KERNEL_TMA_NARROW = 5,
+    MNAD_KERNEL_RESIDENT = 6
 };
 
 typedef struct mnad_options {
@@ -266,16 +272,19 @@ MNAD_API int mnad_plan_destroy(mnad_plan* plan);
  * and the algorithmic HBM bytes of those updates. */
 MNAD_API int mnad_plan_work(const mnad_plan* plan, double* point_updates, double* algorithmic_bytes);
 /* Device time of the last run (ms, CUDA events on the plan's stream) and the
- * device time spent in step kernels only. */
+ * device time spent in step kernels only.  step_launches counts time steps per
+ * launch group (two of the two-step kernel's are one); the on-chip kernel runs
+ * many in a launch: mnad_plan_launches has the step-kernel launches issued. */
 MNAD_API int mnad_plan_timing(const mnad_plan* plan, double* run_ms, double* step_ms, int* step_launches);
+MNAD_API int mnad_plan_launches(const mnad_plan* plan, int* kernel_launches);
 /* The last run split by phase: device time (ms) and algorithmic bytes of the
  * forwards (phase 1) and of the adjoints (phase 3; with checkpointing this
  * phase also holds the background recomputation). */
 MNAD_API int mnad_plan_phases(const mnad_plan* plan, double* forward_ms, double* forward_bytes, double* adjoint_ms,
                               double* adjoint_bytes);
-/* Step kernel (MNAD_KERNEL_DIRECT, _TMA, _TMA_NARROW or _TMA2) that the
+/* Step kernel (MNAD_KERNEL_DIRECT, _TMA, _TMA_NARROW, _TMA2 or _RESIDENT) that the
  * forward phase and the adjoint phase of the plan run, for the launch group
- * with the most tiles (after MNAD_KERNEL_TUNE's trials, once the plan has
+ * with the most points (after MNAD_KERNEL_TUNE's trials, once the plan has
  * run).  -1 where a phase has no propagation. */
 MNAD_API int mnad_plan_kernels(const mnad_plan* plan, int* forward_kernel, int* adjoint_kernel);
 /* Stack of the plan's RTM shots after mnad_plan_run, formed in FP64 on the

@@ -198,6 +198,7 @@ MNAD_API int mnad_fwd_fields(mnad_context* ctx, double dx, double xs, const doub
         p.build(c);
         Batch b(c, tc);
         b.add(&p);
+        b.expect_window(nt / (nkeep + 1));
         b.finalize();
         b.start();
         const size_t N = (size_t)nz * nx;
@@ -426,7 +427,7 @@ struct mnad_plan {
     double pts = 0, bytes = 0;
     double bytes_fwd = 0, bytes_adj = 0;        // phase 1 / phase 3 (with the recomputation)
     float run_ms = 0, step_ms = 0, fwd_ms = 0, adj_ms = 0;
-    int launches = 0;
+    int launches = 0, issued = 0;      // of the last run: time steps (step_launches), step-kernel launches
     // run once and destroyed (mnad_run_jobs): launch the steps directly --
     // capturing and instantiating a graph of thousands of launches costs more
     // than it saves on a single run, and direct launches overlap the GPU work
@@ -454,7 +455,7 @@ static Prop* add_prop(mnad_plan& P, const mnad_job& j, int mode, const double* v
 // that image with exactly those snapshots.  Each propagation advances only in
 // its own window of global steps (s_begin, s_end), with s_off chosen so its
 // local step continues where it stands and its time level keeps the parity of
-// the global step.  Returns the number of step launches.
+// the global step.  Returns the number of time steps launched.
 static int run_segments(mnad_plan& P)
 {
     Context& c = *P.ctx;
@@ -484,7 +485,7 @@ static int run_segments(mnad_plan& P)
             L = std::max(L, len);
         }
         P.recomp->refresh_descs();
-        P.recomp->advance(R, R + L);
+        P.issued += P.recomp->advance(R, R + L);
         launches += L;
         R += L + (L & 1);
         L = 0;
@@ -505,7 +506,7 @@ static int run_segments(mnad_plan& P)
             L = std::max(L, (sa & 1) + len);
         }
         P.phase3->refresh_descs();
-        P.phase3->advance(R, R + L);
+        P.issued += P.phase3->advance(R, R + L);
         launches += L;
         R += L + (L & 1);
     }
@@ -609,7 +610,14 @@ MNAD_API int mnad_plan_create(mnad_context* ctx, const mnad_job* jobs, int njobs
                 P->bytes += b->algorithmic_bytes();
                 P->bytes_adj += b->algorithmic_bytes();
             }
-        if (P->ckpt) P->recomp->finalize();
+        if (P->ckpt) {
+            int window = INT_MAX;                       // the segments of run_segments
+            for (int k = 0; k < njobs; ++k)
+                if (P->fwd_bg[k]) window = std::min(window, P->ck_C[k]);
+            P->recomp->expect_window(window);
+            P->phase3->expect_window(window);
+            P->recomp->finalize();
+        }
         P->phase1->finalize();
         P->phase3->finalize();
         for (auto& e : P->ev) MNAD_CK(cudaEventCreate(&e));
@@ -637,9 +645,14 @@ MNAD_API int mnad_plan_run(mnad_plan* P)
             MNAD_CK(cudaGetLastError());
         }
         MNAD_CK(cudaEventRecord(P->ev[2], c.stream));
+        P->issued = P->phase1->launched();
         int seg_launches = 0;
-        if (P->ckpt) seg_launches = run_segments(*P);
-        else P->phase3->run(g);
+        if (P->ckpt) {
+            seg_launches = run_segments(*P);
+        } else {
+            P->phase3->run(g);
+            P->issued += P->phase3->launched();
+        }
         MNAD_CK(cudaEventRecord(P->ev[3], c.stream));
         MNAD_CK(cudaEventSynchronize(P->ev[3]));
         float a = 0, b = 0, t = 0;
@@ -714,6 +727,14 @@ MNAD_API int mnad_plan_timing(const mnad_plan* P, double* run_ms, double* step_m
         if (run_ms) *run_ms = P->run_ms;
         if (step_ms) *step_ms = P->step_ms;
         if (launches) *launches = P->launches;
+    });
+}
+
+MNAD_API int mnad_plan_launches(const mnad_plan* P, int* kernel_launches)
+{
+    return guard([&] {
+        need(P && kernel_launches, "NULL argument");
+        *kernel_launches = P->issued;
     });
 }
 

@@ -122,6 +122,8 @@ struct __align__(16) PropDesc {
     int snap_stage;          // forward with the FP16 codec: every snapshot is
                              // written in FP32 to one staging slot, then encoded
     const float* snap_scale; // per-snapshot scale (FP16 codec), may be null
+    void* enc;               // forward with the FP16 codec: the encoded snapshots [nsnap][nint]
+    float* enc_scale;        // and their scales (the on-chip kernel encodes them itself)
     int snap_col0;           // snapshot column (0-based) held in the first slot of `snap`
     int snap_cols;           // slots of `snap`: a forward writes, an adjoint reads only
                              // columns snap_col0 .. snap_col0 + snap_cols - 1
@@ -161,6 +163,23 @@ struct StepArgs {
     int s;                 // global step index
     unsigned* status;      // launch-wide status word (ST_TIMEOUT: the launch did not finish its tiles)
     unsigned spin_limit;   // polls of a bounded barrier wait before it gives up (persistent kernels; set by the host, > 0)
+};
+
+// Arguments of one launch of the on-chip kernel: steps s0 .. s1-1 of
+// consecutive propagations of one (dx, dz) group, npatch CTAs each.
+struct ResArgs {
+    Coefs2 coef2;
+    const PropDesc* props;         // the first propagation of the launch
+    const int4* patches;           // {j0, nj, i0, ni}, band by band (mnad_resident.h)
+    const int* band_first;         // first patch of each band, and npatch
+    uint4* words;                  // published cells [propagation][level parity][patch][slot], tags zeroed
+    uint4* peaks;                  // FP16 codec: {largest |d2u| of a snapshot, -, -, its number} [propagation]
+                                   // [number parity][patch], zeroed
+    int npatch, nbands, slots;
+    int comm;                      // threads of a CTA that do the exchange (the last ones)
+    int s0, s1;
+    unsigned* status;
+    unsigned spin_limit;
 };
 
 // Neighbourhood of one point for the three fields.  Naming: <f><z><x> with
@@ -295,6 +314,18 @@ __device__ __forceinline__ float snap_decode(const void* base, int codec, size_t
     if (codec == CODEC_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[i]);
     if (codec == CODEC_F16) return __half2float(static_cast<const __half*>(base)[i]) * scale;
     return static_cast<const float*>(base)[i];
+}
+
+// Power-of-two scale s of an FP16 snapshot, chosen from its largest |x| = mx so
+// that mx/s < 2^14 (no saturation; the scale multiply is exact), and 1/s.
+// Arrays whose maximum is below 2^-100 keep s = 2^-114, so 1/s stays finite.
+__device__ __forceinline__ void f16_scale(float mx, float& s, float& inv)
+{
+    int e = 0;
+    frexpf(mx, &e);                                   // mx = f * 2^e, 0.5 <= f < 1
+    e = max(e, -100);                                 // tiny maxima: keep 2^(14-e) finite
+    s = mx > 0.0f ? ldexpf(1.0f, e - 14) : 1.0f;
+    inv = mx > 0.0f ? ldexpf(1.0f, 14 - e) : 1.0f;
 }
 
 // The FP64 value of a float, from its IEEE-754 fields with integer

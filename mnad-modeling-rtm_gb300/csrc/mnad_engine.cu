@@ -98,6 +98,15 @@ void Context::release(void* p, size_t bytes)
 
 void Context::sync() { MNAD_CK(cudaStreamSynchronize(stream)); }
 
+std::shared_ptr<const ResPlan> Context::resident_plan(int nz, int nx, int d, int ncta)
+{
+    const auto key = std::make_tuple(nz, nx, d, ncta);
+    auto it = res_plans.find(key);
+    if (it != res_plans.end()) return it->second;
+    if (res_plans.size() >= 256) res_plans.clear();
+    return res_plans[key] = std::make_shared<const ResPlan>(res_plan(nz, nx, d, ncta));
+}
+
 unsigned Context::take_status()
 {
     unsigned s = 0;
@@ -402,6 +411,8 @@ void Prop::build(Context& ctx)
             D.codec = CODEC_F32;
             D.snap_stage = 1;
             D.snap_cols = 1;
+            D.enc = wf.snap.get();
+            D.enc_scale = wf.scale.as<float>();
         }
         if (s.mode == MODE_FWD) {
             D.illum = wf.illum.as<double>();
@@ -610,6 +621,18 @@ void Batch::finalize()
     }
     for (auto& g : groups_) {
         g->kind = pick_kind(*g);
+        if (tc_.kind == MNAD_KERNEL_AUTO && setup_resident(*g)) {
+            std::vector<PropDesc> descs;
+            for (Prop* p : g->props) {
+                p->desc.tile_base = (int)descs.size() * g->tiles_per_prop;
+                descs.push_back(p->desc);
+                all.push_back(p->desc);
+            }
+            ntiles_ += g->ntiles;
+            g->desc = DevMem(&ctx_, descs.size() * sizeof(PropDesc));
+            upload(ctx_, g->desc.get(), descs.data(), descs.size() * sizeof(PropDesc));
+            continue;
+        }
         const bool tma2 = g->kind == MNAD_KERNEL_TMA2;
         const bool narrow = g->kind == MNAD_KERNEL_TMA_NARROW;
         const bool tma = g->kind == MNAD_KERNEL_TMA || tma2 || narrow;
@@ -814,9 +837,113 @@ void Batch::tune()
     finalize();
 }
 
-void Batch::launch_step(int s, int slot)
+// (c, c) pairs of the coefficients, the negated combinations' ones negated (Coefs2).
+static Coefs2 pair_coefs(const Coefs& c)
 {
-    for (size_t gi = 0; gi < groups_.size(); ++gi) launch_group(gi, s, slot);
+    Coefs2 c2;
+    for (int k = 0; k < NCOEF; ++k) {
+        const float sa = k == K_UV_X1 ? -1.0f : 1.0f, sb = (k == K_UV_X1 || k == K_UV_D) ? -1.0f : 1.0f;
+        c2.alpha[k] = make_float2(sa * c.alpha[k], sa * c.alpha[k]);
+        c2.beta[k] = make_float2(sb * c.beta[k], sb * c.beta[k]);
+    }
+    return c2;
+}
+
+static auto resident_kernel(const LaunchGroup& g)
+{
+    return g.res->small ? (g.point_order ? step_resident_small_point : step_resident_small)
+                        : (g.point_order ? step_resident_point : step_resident);
+}
+
+// The on-chip kernel for a group that the AUTO rule has given g.kind: false
+// where a propagation's state does not fit the SMs, or the device memory for
+// the published cells is not to be had (the group then runs g.kind).
+bool Batch::setup_resident(LaunchGroup& g)
+{
+    const int n = (int)g.props.size(), S = ctx_.num_sms;
+    if (n == 0 || shortest_run() < RES_MIN_RUN) return false;
+    // Propagations of like lengths share launches (a launch runs as long as its
+    // longest).  How many: the split with the shortest estimated run.
+    std::stable_sort(g.props.begin(), g.props.end(), [](const Prop* a, const Prop* b) { return a->spec.nt > b->spec.nt; });
+    const double quads = (double)((g.nz + 3) / 4) * g.nx;
+    const double cost = quads + RES_STRIP_COST * 2.0 * g.d * (g.nz + g.nx) / 4;
+    std::vector<std::pair<double, int>> waves;
+    for (int m = 1; m <= std::min(n, S); ++m) {
+        const double k = std::min<double>(S / m, std::max(1.0, quads / RES_MIN_QUADS));
+        double steps = 0;
+        for (int p = 0; p < n; p += m) steps += g.props[p]->spec.nt;
+        waves.emplace_back(steps * (RES_STEP_US + RES_QUAD_US * cost / k), m);
+    }
+    std::sort(waves.begin(), waves.end());
+    for (const auto& w : waves) {
+        const auto plan = ctx_.resident_plan(g.nz, g.nx, g.d, S / w.second);
+        const ResPlan& p = *plan;
+        if (!p.ok()) {
+            if (w.second == 1) return false;       // not even with every SM
+            continue;
+        }
+        const int np = (int)p.patches.size();
+        try {
+            // the split, the snapshots' maxima, the published cells
+            g.res_mem = DevMem(&ctx_, (RES_TABLE + (size_t)w.second * np * 2 * (1 + (np > 1 ? p.slots : 0))) * sizeof(uint4));
+        } catch (const Error& e) {
+            if (e.code == MNAD_E_BUDGET || e.code == MNAD_E_OOM) return false;
+            throw;
+        }
+        static_assert(sizeof(ResPatch) == sizeof(int4), "patches travel as int4");
+        std::vector<int> table(4 * RES_TABLE, 0);
+        std::memcpy(table.data(), p.patches.data(), np * sizeof(ResPatch));
+        std::copy(p.band_first.begin(), p.band_first.end(), table.begin() + 4 * RES_MAX_PATCHES);
+        upload(ctx_, g.res_mem.get(), table.data(), table.size() * sizeof(int));
+        g.res = plan;
+        g.wave = w.second;
+        g.point_order = g.kind == MNAD_KERNEL_DIRECT;
+        g.kind = MNAD_KERNEL_RESIDENT;
+        MNAD_CK(cudaFuncSetAttribute(resident_kernel(g), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM_LIMIT - 1024));
+        g.tiles_per_prop = np;
+        g.ntiles = np * n;
+        return true;
+    }
+    return false;
+}
+
+int Batch::launch_resident(LaunchGroup& g, int s0, int s1)
+{
+    int launches = 0;
+    ResArgs a;
+    a.coef2 = pair_coefs(g.coefs);
+    a.patches = g.res_mem.as<int4>();
+    a.band_first = reinterpret_cast<const int*>(a.patches + RES_MAX_PATCHES);
+    a.npatch = (int)g.res->patches.size();
+    a.nbands = (int)g.res->band_first.size() - 1;
+    a.slots = g.res->slots;
+    a.comm = g.res->comm;
+    a.s0 = s0;
+    a.s1 = s1;
+    a.status = ctx_.d_status;
+    a.spin_limit = ctx_.wait_limit ? ctx_.wait_limit : SPIN_LIMIT_DEFAULT;
+    for (size_t p0 = 0; p0 < g.props.size(); p0 += g.wave) {
+        const int n = (int)std::min<size_t>(g.wave, g.props.size() - p0);
+        a.props = g.desc.as<PropDesc>() + p0;
+        // no cell and no maximum of an earlier launch may pass for one of this
+        a.peaks = g.res_mem.as<uint4>() + RES_TABLE;
+        a.words = a.peaks + (size_t)n * a.npatch * 2;
+        MNAD_CK(cudaMemsetAsync(a.peaks, 0, (size_t)n * a.npatch * 2 * (1 + (a.npatch > 1 ? a.slots : 0)) * sizeof(uint4),
+                                ctx_.stream));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;      // the CTAs wait for one another
+        at[0].val.cooperative = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(n * a.npatch);
+        cfg.blockDim = dim3(g.res->threads);
+        cfg.dynamicSmemBytes = g.res->smem;
+        cfg.stream = ctx_.stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        MNAD_CK(cudaLaunchKernelEx(&cfg, resident_kernel(g), a));
+        ++launches;
+    }
+    return launches;
 }
 
 void Batch::launch_group(size_t gi, int s, int slot)
@@ -827,11 +954,7 @@ void Batch::launch_group(size_t gi, int s, int slot)
         if (g->kind == MNAD_KERNEL_TMA2 && (s & 1)) return;   // step s ran in the launch at s - 1
         StepArgs a;
         a.coef = g->coefs;
-        for (int k = 0; k < NCOEF; ++k) {
-            const float sa = k == K_UV_X1 ? -1.0f : 1.0f, sb = (k == K_UV_X1 || k == K_UV_D) ? -1.0f : 1.0f;
-            a.coef2.alpha[k] = make_float2(sa * g->coefs.alpha[k], sa * g->coefs.alpha[k]);
-            a.coef2.beta[k] = make_float2(sb * g->coefs.beta[k], sb * g->coefs.beta[k]);
-        }
+        a.coef2 = pair_coefs(g->coefs);
         a.props = g->desc.as<PropDesc>();
         a.tile_prop = g->tile_prop.as<int>();
         a.tmaps = g->tmaps.get();
@@ -869,18 +992,21 @@ void Batch::start()
 
 void Batch::encode_snapshots(int s)
 {
-    for (Prop* p : props_) {
-        const PropSpec& sp = p->spec;
-        if (sp.mode != MODE_FWD || !sp.wf || sp.wf->codec != MNAD_SNAP_F16 || sp.T <= 0) continue;
-        const int tt = s - p->desc.s_off + 1;
-        if (tt < 1 || tt > sp.nt || tt % sp.T != 0 || tt / sp.T > sp.wf->nsnap) continue;
-        const int k = tt / sp.T - 1;
-        Wavefield& wf = *sp.wf;
-        const size_t n = wf.nint;
-        const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx_.num_sms * 4);
-        f16_absmax<<<blocks, 256, 0, ctx_.stream>>>(wf.stage.as<float>(), n, wf.maxbits.as<unsigned>() + k);
-        f16_encode<<<blocks, 256, 0, ctx_.stream>>>(wf.stage.as<float>(), n, wf.maxbits.as<unsigned>() + k,
-                                                    wf.snap.as<__half>() + (size_t)k * n, wf.scale.as<float>() + k);
+    for (const auto& g : groups_) {
+        if (g->kind == MNAD_KERNEL_RESIDENT) continue;      // encodes them itself
+        for (Prop* p : g->props) {
+            const PropSpec& sp = p->spec;
+            if (sp.mode != MODE_FWD || !sp.wf || sp.wf->codec != MNAD_SNAP_F16 || sp.T <= 0) continue;
+            const int tt = s - p->desc.s_off + 1;
+            if (tt < 1 || tt > sp.nt || tt % sp.T != 0 || tt / sp.T > sp.wf->nsnap) continue;
+            const int k = tt / sp.T - 1;
+            Wavefield& wf = *sp.wf;
+            const size_t n = wf.nint;
+            const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx_.num_sms * 4);
+            f16_absmax<<<blocks, 256, 0, ctx_.stream>>>(wf.stage.as<float>(), n, wf.maxbits.as<unsigned>() + k);
+            f16_encode<<<blocks, 256, 0, ctx_.stream>>>(wf.stage.as<float>(), n, wf.maxbits.as<unsigned>() + k,
+                                                        wf.snap.as<__half>() + (size_t)k * n, wf.scale.as<float>() + k);
+        }
     }
 }
 
@@ -934,9 +1060,36 @@ void Batch::refresh_descs()
     if (!all.empty()) upload(ctx_, d_all_desc_.get(), all.data(), all.size() * sizeof(PropDesc));
 }
 
-void Batch::advance(int s0, int s1)
+// Steps between two returns to the host, as far as it is known before the run.
+int Batch::shortest_run() const
 {
-    if (ntiles_ == 0) return;
+    int run = window_;
+    for (const Prop* p : props_) {
+        if (p->energy.get()) run = std::min(run, p->spec.energy_every);
+        if (p->ckpt.saving && p->ckpt.C > 0) run = std::min(run, p->ckpt.C);
+    }
+    return run;
+}
+
+bool Batch::hook_due(int s) const
+{
+    for (const auto& g : groups_)
+        for (const Prop* p : g->props) {
+            const PropSpec& sp = p->spec;
+            const int done = s - p->desc.s_off + 1;         // its steps done after global step s
+            if (done < 1 || done > sp.nt) continue;
+            if (g->kind != MNAD_KERNEL_RESIDENT && sp.mode == MODE_FWD && sp.wf && sp.wf->codec == MNAD_SNAP_F16 && sp.T > 0 &&
+                done % sp.T == 0)
+                return true;
+            if (p->energy.get() && done % sp.energy_every == 0) return true;
+            if (p->ckpt.saving && p->ckpt.C > 0 && done % p->ckpt.C == 0) return true;
+        }
+    return false;
+}
+
+int Batch::advance(int s0, int s1)
+{
+    if (ntiles_ == 0) return 0;
     bool f16 = false, en = false, ck = false;
     for (Prop* p : props_) {
         f16 |= p->spec.mode == MODE_FWD && p->spec.wf && p->spec.wf->codec == MNAD_SNAP_F16;
@@ -948,13 +1101,33 @@ void Batch::advance(int s0, int s1)
         const size_t need = reserve_counters(s1 - s0);
         MNAD_CK(cudaMemsetAsync(d_counters_.get(), 0, need, ctx_.stream));
     }
-    for (int s = s0; s < s1; ++s) {
-        launch_step(s, s - s0);
-        if (f16) encode_snapshots(s);
-        if (en) energy_after(s);
-        if (ck) checkpoint_after(s);
+    int launches = 0;
+    for (int s = s0, e; s < s1; s = e) {
+        // up to the next step that host work follows
+        e = s1;
+        if (f16 || en || ck)
+            for (e = s + 1; e < s1 && !hook_due(e - 1);) ++e;
+        for (int t = s; t < e; ++t)
+            for (size_t gi = 0; gi < groups_.size(); ++gi)
+                if (groups_[gi]->kind != MNAD_KERNEL_RESIDENT) {
+                    launch_group(gi, t, t - s0);
+                    launches += groups_[gi]->kind != MNAD_KERNEL_TMA2 || !(t & 1);
+                }
+        for (auto& g : groups_)
+            if (g->kind == MNAD_KERNEL_RESIDENT) launches += launch_resident(*g, s, e);
+        if (f16) encode_snapshots(e - 1);
+        if (en) energy_after(e - 1);
+        if (ck) checkpoint_after(e - 1);
     }
     MNAD_CK(cudaGetLastError());
+    return launches;
+}
+
+bool Batch::all_resident() const
+{
+    for (const auto& g : groups_)
+        if (g->kind != MNAD_KERNEL_RESIDENT) return false;
+    return true;
 }
 
 bool Batch::has_tma() const
@@ -983,10 +1156,11 @@ int Batch::step_launches() const
 
 int Batch::main_kind() const
 {
-    int kind = -1, most = 0;
+    int kind = -1;
+    double most = 0;
     for (const auto& g : groups_)
-        if (g->ntiles > most) {
-            most = g->ntiles;
+        if (g->points() > most) {
+            most = g->points();
             kind = g->kind;
         }
     return kind;
@@ -1011,7 +1185,7 @@ bool Batch::has_step_hooks() const
 void Batch::tick(int K, bool use_graph)
 {
     if (ntiles_ == 0 || K <= 0) return;
-    if (!use_graph || has_step_hooks()) {
+    if (!use_graph || has_step_hooks() || all_resident()) {    // a few launches need no graph
         advance(0, K);
         return;
     }
@@ -1042,11 +1216,12 @@ void Batch::run(bool use_graph)
             graph_ = nullptr;
         }
     }
-    auto body = [&]() {
+    auto body = [&] {
         start();
-        advance(0, nsteps_);
+        launched_ = advance(0, nsteps_);
     };
-    if (!use_graph) {
+    // the state's memsets are most of the launches of an all-resident run; few need no graph
+    if (!use_graph || (all_resident() && props_.size() <= 16)) {
         body();
         MNAD_CK(cudaGetLastError());
         return;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <map>
 #include <tuple>
@@ -13,6 +14,7 @@
 
 #include "../../include/mnad.h"
 #include "mnad_device.cuh"
+#include "mnad_resident.h"
 
 namespace mnad {
 
@@ -70,6 +72,9 @@ struct Context {
     std::map<int, std::unique_ptr<Wavefield>> wavefields;
     // MNAD_KERNEL_TUNE: measured step kernel per (nz, nx, d_pml, propagations per launch)
     std::map<std::tuple<int, int, int, int>, int> kernel_choice;
+    // splits of a grid over CTAs for the on-chip kernel, by (nz, nx, d_pml, CTAs); bounded
+    std::map<std::tuple<int, int, int, int>, std::shared_ptr<const ResPlan>> res_plans;
+    std::shared_ptr<const ResPlan> resident_plan(int nz, int nx, int d, int ncta);
     std::vector<double> last_energy;  // energy history of the last drop-in forward
 
     explicit Context(int dev, size_t budget_bytes);
@@ -81,7 +86,8 @@ struct Context {
 };
 
 // Step-kernel choice of a batch: MNAD_KERNEL_DIRECT, MNAD_KERNEL_TMA,
-// MNAD_KERNEL_AUTO (per launch group: the TMA kernel once a launch has
+// MNAD_KERNEL_AUTO (per launch group: the on-chip kernel where the state of a
+// propagation fits the SMs; else the TMA kernel once a launch has
 // AUTO_TMA_TILES_PER_CTA of its tiles for each resident CTA, the direct
 // kernel below) or MNAD_KERNEL_TUNE (per launch group, measured on the
 // batch's own propagations at its first run; Batch::tune).
@@ -99,6 +105,14 @@ constexpr double AUTO_TMA_TILES_PER_CTA = 2.25;
 // the grid, the 64 x 16 tiles above it (between two measured grids: 8 % and
 // 22 %).
 constexpr double AUTO_NARROW_STRIP_SHARE = 0.15;
+// The on-chip kernel's step: the exchange between patches, and a 4-row
+// group of the costliest CTA (used to choose how many propagations share a launch).
+constexpr double RES_STEP_US = 1.2, RES_QUAD_US = 0.0033;
+// Runs of fewer steps between two returns to the host do not pay for loading
+// and storing the state (break-even about 4 steps: a shot of 96 x 112, energy
+// every step 8.0 ms on chip, 4.3 ms step by step; every 4 steps 2.6 and 2.8 ms;
+// every 8 steps 1.7 and 2.6 ms).
+constexpr int RES_MIN_RUN = 6;
 constexpr int TUNE_WARMUP = 2, TUNE_STEPS = 8;
 
 // Receivers of one propagation bucketed by TMA_TZ x TMA_TX tile and, within a
@@ -179,6 +193,14 @@ struct LaunchGroup {
     DevMem desc, tile_prop, tmaps, tile_info;
     int ntiles = 0;                    // tiles of one launch (of the group's kernel)
     int ntz = 0, tiles_per_prop = 0;   // tiling of the group's kernel
+    // MNAD_KERNEL_RESIDENT: the grid's split, propagations per launch, whether
+    // the one-thread-per-point kernel's rounding is kept, the split on
+    // the device with the published cells of one launch
+    std::shared_ptr<const ResPlan> res;
+    int wave = 0;
+    bool point_order = false;
+    DevMem res_mem;
+    double points() const { return (double)nz * nx * props.size(); }
 };
 
 // Propagations that advance together: one launch per geometry group and step
@@ -197,8 +219,9 @@ public:
     // per group; choices are cached in the context.  The trial steps leave
     // no trace: run() starts from start(), which resets what they touched.
     void tune();
+    void expect_window(int k) { window_ = k; }   // advance() and tick() will run about k steps at a time (before finalize)
     void start();                      // zero all state and seed the sources (async)
-    void advance(int s0, int s1);      // launch global steps s0..s1-1 (async)
+    int advance(int s0, int s1);       // launch global steps s0..s1-1 (async); step-kernel launches issued
     void refresh_descs();              // re-upload the descriptors after host-side changes
     // Global steps 0..K-1 (async), as one CUDA graph replayed tick after tick
     // when `use_graph` and no propagation needs per-step host work; callers
@@ -207,17 +230,24 @@ public:
     bool has_step_hooks() const;       // FP16 snapshot encodes, energy or checkpoints per step
     bool has_tma() const;              // a group runs the TMA kernel
     int launches_per_step() const;     // step-kernel launches of one time step
-    int step_launches() const;         // step-kernel launches of a whole run (run())
+    int step_launches() const;         // time steps of a whole run (run()), per launch group, two-step launches once
+    int launched() const { return launched_; }   // step-kernel launches of the last run()
     int group_kind_count(int kind) const;   // launch groups running that kernel
-    int main_kind() const;             // kernel of the group with the most tiles (-1: no group)
+    int main_kind() const;             // kernel of the group with the most points (-1: no group)
     int group_kind(size_t g) const { return groups_[g]->kind; }
     size_t groups() const { return groups_.size(); }
     int steps() const { return nsteps_; }
     int tiles() const { return ntiles_; }
     const std::vector<Prop*>& props() const { return props_; }
 private:
-    void launch_step(int s, int slot);
+    int launched_ = 0;
+    int window_ = INT_MAX;
+    int shortest_run() const;
     void launch_group(size_t gi, int s, int slot);
+    int launch_resident(LaunchGroup& g, int s0, int s1);
+    bool setup_resident(LaunchGroup& g);
+    bool hook_due(int s) const;        // per-step host work follows step s
+    bool all_resident() const;         // every group runs the on-chip kernel
     int pick_kind(const LaunchGroup& g) const;
     bool depth2_allowed(const LaunchGroup& g) const;
     size_t reserve_counters(int nsteps);   // tile counters for nsteps steps (bytes used)

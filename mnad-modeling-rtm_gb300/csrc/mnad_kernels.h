@@ -46,6 +46,13 @@ size_t step_tma_narrow_smem_bytes();
 // Two time steps (A.s even, and A.s + 1) per launch; see mnad_step_tma2.cu.
 __global__ void step_tma2(const __grid_constant__ StepArgs A);
 size_t step_tma2_smem_bytes();
+// Steps s0 .. s1-1 in one cooperative launch, state on chip; see
+// mnad_step_resident.cu.  step_resident rounds as the persistent kernels,
+// step_resident_point as step_direct; _small for plans of small patches only.
+__global__ void step_resident(const __grid_constant__ ResArgs A);
+__global__ void step_resident_point(const __grid_constant__ ResArgs A);
+__global__ void step_resident_small(const __grid_constant__ ResArgs A);
+__global__ void step_resident_small_point(const __grid_constant__ ResArgs A);
 __global__ void build_r(const double* __restrict__ v, int nz, int nx, double dt, int adjoint,
                         float* __restrict__ r, int ld);
 __global__ void seed_sources(const PropDesc* __restrict__ props, int n);

@@ -289,6 +289,7 @@ void mnad_server::loop()
                     batch->add(j->fwd_true.get());
                     if (j->fwd_bg) batch->add(j->fwd_bg.get());
                 }
+                batch->expect_window(K);
                 batch->finalize();
                 dirty = false;
             }

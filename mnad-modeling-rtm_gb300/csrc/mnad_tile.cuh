@@ -215,6 +215,10 @@ __device__ __forceinline__ float2 pr(float a, float b) { return make_float2(a, b
 // between rows: e.g. the diagonal sum of point k is S[k] + S[k+2] and the odd
 // diagonal of Avu_gen.m is D[k] + D[k+2].  Per point the operations, their
 // order and their rounding are those of mnad_update.
+// POINT_ORDER takes the diagonal sums in the order of mnad_update (the
+// one-thread-per-point kernel) instead, point for point and bit for bit; the
+// self terms, the rows and their coefficients are common to both.
+template <bool POINT_ORDER = false>
 __device__ __forceinline__ void mnad_update_pairs(const Coefs2& K, const Window& win, const float* rr, float2* su,
                                                   float2* sv, float2* sw)
 {
@@ -258,26 +262,55 @@ __device__ __forceinline__ void mnad_update_pairs(const Coefs2& K, const Window&
         const float2 uzs = pr(U[k] + U[k + 2], U[k + 1] + U[k + 3]);
         const float2 vzs = pr(V[k] + V[k + 2], V[k + 1] + V[k + 3]);
         const float2 wzs = pr(W[k] + W[k + 2], W[k + 1] + W[k + 3]);
+        // diagonal sums of a field in point order: A = (z-1,x-1) + (z+1,x+1),
+        // B = (z+1,x-1) + (z-1,x+1); column sums Z = F(z-1) + F(z+1)
+        constexpr int R = Window::R;
+        auto diag_a = [k](const float (*F)[R]) { return pr(F[0][k] + F[2][k + 2], F[0][k + 1] + F[2][k + 3]); };
+        auto diag_b = [k](const float (*F)[R]) { return pr(F[0][k + 2] + F[2][k], F[0][k + 3] + F[2][k + 1]); };
+        auto zsum = [k](const float* F) { return pr(F[k] + F[k + 2], F[k + 1] + F[k + 3]); };
         // U combinations (Auu, Avu, Awu)
         const float2 dUz = psub(uzs, u2), dUx = psub(SUp[m], u2);
-        const float2 dUd = psub(pr(SU[k] + SU[k + 2], SU[k + 1] + SU[k + 3]), padd(u2, u2));
         const float2 uLx = DUp[m], uLz = pr(U[k] - U[k + 2], U[k + 1] - U[k + 3]);
-        const float2 uDx = pr(DU[k] + DU[k + 2], DU[k + 1] + DU[k + 3]);
         const float2 uDz = pr(SU[k] - SU[k + 2], SU[k + 1] - SU[k + 3]);
+        float2 dUd, uDx;
+        if constexpr (POINT_ORDER) {
+            dUd = psub(padd(diag_a(win.u), diag_b(win.u)), padd(u2, u2));
+            uDx = psub(zsum(win.u[0]), zsum(win.u[2]));
+        } else {
+            dUd = psub(pr(SU[k] + SU[k + 2], SU[k + 1] + SU[k + 3]), padd(u2, u2));
+            uDx = pr(DU[k] + DU[k + 2], DU[k + 1] + DU[k + 3]);
+        }
         // V combinations (Avv, Auv, Awv); vX1 and vDx enter with negative sign
         const float2 dVz = psub(vzs, v2), dVx = psub(SVp[m], v2);
-        const float2 dVd = psub(pr(SV[k] + SV[k + 2], SV[k + 1] + SV[k + 3]), padd(v2, v2));
-        const float2 nvX1 = DVp[m], nvDx = pr(DV[k] + DV[k + 2], DV[k + 1] + DV[k + 3]);
+        const float2 nvX1 = DVp[m];
         const float2 vX2 = psub(pr(win.v2m[k], win.v2m[k + 1]), pr(win.v2p[k], win.v2p[k + 1]));
-        const float2 vXZ = pr(DV[k] - DV[k + 2], DV[k + 1] - DV[k + 3]);
+        float2 dVd, nvDx, vXZ;
+        if constexpr (POINT_ORDER) {
+            const float2 vA = diag_a(win.v), vB = diag_b(win.v);
+            dVd = psub(padd(vA, vB), padd(v2, v2));
+            nvDx = psub(zsum(win.v[0]), zsum(win.v[2]));
+            vXZ = psub(vA, vB);
+        } else {
+            dVd = psub(pr(SV[k] + SV[k + 2], SV[k + 1] + SV[k + 3]), padd(v2, v2));
+            nvDx = pr(DV[k] + DV[k + 2], DV[k + 1] + DV[k + 3]);
+            vXZ = pr(DV[k] - DV[k + 2], DV[k + 1] - DV[k + 3]);
+        }
         // W combinations (Aww, Auw, Avw)
         const float2 wzm2 = m == 0 ? pr(win.wz[0], W[0]) : pr(W[1], W[2]);
         const float2 wzp2 = m == 0 ? pr(W[3], W[4]) : pr(W[5], win.wz[1]);
         const float2 dWz = psub(wzs, w2), dWx = psub(SWp[m], w2);
-        const float2 dWd = psub(pr(SW[k] + SW[k + 2], SW[k + 1] + SW[k + 3]), padd(w2, w2));
         const float2 wZ1 = pr(W[k + 2] - W[k], W[k + 3] - W[k + 1]);
         const float2 wDz = pr(SW[k + 2] - SW[k], SW[k + 3] - SW[k + 1]);
-        const float2 wZ2 = psub(wzm2, wzp2), wXZ = pr(DW[k] - DW[k + 2], DW[k + 1] - DW[k + 3]);
+        const float2 wZ2 = psub(wzm2, wzp2);
+        float2 dWd, wXZ;
+        if constexpr (POINT_ORDER) {
+            const float2 wA = diag_a(win.w), wB = diag_b(win.w);
+            dWd = psub(padd(wA, wB), padd(w2, w2));
+            wXZ = psub(wA, wB);
+        } else {
+            dWd = psub(pr(SW[k] + SW[k + 2], SW[k + 1] + SW[k + 3]), padd(w2, w2));
+            wXZ = pr(DW[k] - DW[k + 2], DW[k + 1] - DW[k + 3]);
+        }
         // nU row
         float2 ra = pmul(a[K_UU_Z], dUz);
         ra = pfma(a[K_UU_X], dUx, ra);
@@ -373,19 +406,29 @@ __device__ __forceinline__ void injection(const PropDesc& P, int tt, int tl, int
 // C_cof.m:6-16 at a z-pair of points: (c1, c2, c3) of a side from the
 // velocities and the distance terms X (X = 0 outside the strip gives exactly
 // 1, 0, 0), in packed FP32x2.  An approximate reciprocal is used for these
-// damping coefficients only.
+// damping coefficients only.  POINT_ORDER rounds as cpml_coefs (fused
+// multiply-adds, IEEE reciprocal) instead.
 struct CpmlC {
     float2 c1, c2, c3;
 };
+template <bool POINT_ORDER = false>
 __device__ __forceinline__ CpmlC cpml_c2(float K, float2 vel, float2 X, float dt)
 {
     const float2 s0 = pmul(pr(K, K), vel);
     const float2 sig = pmul(s0, pmul(X, X));
-    const float2 a = pmul(sig, pr(0.5f * dt, 0.5f * dt));
-    const float2 den = padd(pr(1.0f, 1.0f), a);
-    const float2 inv = pr(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
     CpmlC c;
-    c.c1 = pmul(psub(pr(1.0f, 1.0f), a), inv);
+    float2 inv;
+    if constexpr (POINT_ORDER) {
+        const float2 hdt = pr(0.5f * dt, 0.5f * dt), one = pr(1.0f, 1.0f);
+        const float2 den = pfma(sig, hdt, one);
+        inv = pr(__frcp_rn(den.x), __frcp_rn(den.y));
+        c.c1 = pmul(pfma(pr(-sig.x, -sig.y), hdt, one), inv);
+    } else {
+        const float2 a = pmul(sig, pr(0.5f * dt, 0.5f * dt));
+        const float2 den = padd(pr(1.0f, 1.0f), a);
+        inv = pr(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
+        c.c1 = pmul(psub(pr(1.0f, 1.0f), a), inv);
+    }
     c.c2 = pmul(pmul(pmul(pmul(pr(2.0f, 2.0f), s0), X), pr(dt, dt)), inv);
     c.c3 = pmul(pmul(sig, pr(dt, dt)), inv);
     return c;
@@ -401,8 +444,8 @@ __device__ __forceinline__ float2 cpml_mem2(const CpmlC& c, float2 ih, float2 ih
     const float2 g2 = pmul(pmul(c.c2, ih), gr);
     const float2 hg = pmul(pr(0.5f, 0.5f), g2);
     m3 = pfma(c.c1, m3, hg);
-    m2 = padd(pfma(c.c1, m2, g2), pmul(c.c3, pfma(lap, ih2, pr(-m3.x, -m3.y))));
-    m1 = padd(pfma(c.c1, m1, hg), pmul(c.c3, pfma(pmul(pr(2.0f, 2.0f), lap), ih2, pr(-m2.x, -m2.y))));
+    m2 = pfma(c.c3, pfma(lap, ih2, pr(-m3.x, -m3.y)), pfma(c.c1, m2, g2));
+    m1 = pfma(c.c3, pfma(pmul(pr(2.0f, 2.0f), lap), ih2, pr(-m2.x, -m2.y)), pfma(c.c1, m1, hg));
     return m1;
 }
 

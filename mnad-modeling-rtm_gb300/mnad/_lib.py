@@ -17,6 +17,7 @@ OK, E_ARG, E_OOM, E_CUDA, E_TIMEOUT, E_NOTFOUND, E_NUMERIC, E_BUDGET, E_STATE = 
 SNAP_F32, SNAP_BF16, SNAP_F16 = 0, 1, 2
 PAIR_REFERENCE, PAIR_ALIGNED = 0, 1
 KERNEL_AUTO, KERNEL_DIRECT, KERNEL_TMA, KERNEL_TUNE, KERNEL_TMA2, KERNEL_TMA_NARROW = 0, 1, 2, 3, 4, 5
+KERNEL_RESIDENT = 6        # reported by Plan.kernels(), not an option
 JOB_MODEL, JOB_RTM = 0, 1
 JOB_QUEUED, JOB_RUNNING, JOB_DONE, JOB_FAILED = 0, 1, 2, 3
 
@@ -89,6 +90,7 @@ SIGNATURES = {
     "mnad_plan_destroy": ([_vp], C.c_int),
     "mnad_plan_work": ([_vp, _dp, _dp], C.c_int),
     "mnad_plan_timing": ([_vp, _dp, _dp, C.POINTER(C.c_int)], C.c_int),
+    "mnad_plan_launches": ([_vp, C.POINTER(C.c_int)], C.c_int),
     "mnad_plan_phases": ([_vp, _dp, _dp, _dp, _dp], C.c_int),
     "mnad_plan_kernels": ([_vp, C.POINTER(C.c_int), C.POINTER(C.c_int)], C.c_int),
     "mnad_plan_stack": ([_vp, _dp, _dp, _dp], C.c_int),

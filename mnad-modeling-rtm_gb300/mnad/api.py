@@ -313,6 +313,13 @@ class Plan:
         check(lib().mnad_plan_timing(self._h, C.byref(r), C.byref(s), C.byref(n)))
         return {"run_ms": r.value, "step_ms": s.value, "step_launches": n.value}
 
+    def launches(self):
+        """Step-kernel launches of the last run (the on-chip kernel runs many
+        time steps in one)."""
+        n = C.c_int()
+        check(lib().mnad_plan_launches(self._h, C.byref(n)))
+        return n.value
+
     def phases(self):
         """Device time (ms) and algorithmic bytes of the last run's forward
         phase and adjoint phase."""
@@ -327,6 +334,7 @@ class Plan:
         f, a = C.c_int(), C.c_int()
         check(lib().mnad_plan_kernels(self._h, C.byref(f), C.byref(a)))
         names = {v: k for k, v in _KERNELS.items()}
+        names[_lib.KERNEL_RESIDENT] = "resident"
         return {"forward": names.get(f.value), "adjoint": names.get(a.value)}
 
     def stack(self):
