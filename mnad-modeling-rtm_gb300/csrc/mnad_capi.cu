@@ -17,8 +17,6 @@ struct mnad_context : Context {
     using Context::Context;
 };
 
-static bool use_graph(const Context& c, int nt) { return c.opt.use_graphs != 0 && nt >= 1; }
-
 extern "C" {
 
 MNAD_API int mnad_abi_version(void) { return MNAD_ABI_VERSION; }
@@ -155,7 +153,7 @@ MNAD_API int mnad_fwd_pde_exact(mnad_context* ctx, double dx, double xs, const d
         Batch b(c, tc, p.spec.depth2);
         b.add(&p);
         b.finalize();
-        b.run(use_graph(c, nt));
+        b.run(false);              // one run: launching directly overlaps the GPU, a capture does not
         const size_t nd = (size_t)nt * nr;
         download(c, datau, p.data.get(), nd * sizeof(double));
         if (s.record_vw && datav) download(c, datav, p.datav.get(), nd * sizeof(double));
@@ -289,7 +287,7 @@ MNAD_API int mnad_born_adj(mnad_context* ctx, double dx, double dz, int nt, doub
         Batch b(c, tc, p.spec.depth2);
         b.add(&p);
         b.finalize();
-        b.run(use_graph(c, nt));
+        b.run(false);              // one run: launching directly overlaps the GPU, a capture does not
         const size_t n = p.nint();
         DevMem out(&c, n * sizeof(double));
         scale_f64<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, c.stream>>>(p.image.as<double>(), (double)T, n,

@@ -969,11 +969,28 @@ void Batch::launch_group(size_t gi, int s, int slot)
         a.status = ctx_.d_status;
         a.spin_limit = ctx_.wait_limit ? ctx_.wait_limit : SPIN_LIMIT_DEFAULT;
         const int grid = std::min(g->ntiles, ctx_.num_sms * TMA_CTAS_PER_SM);
-        if (g->kind == MNAD_KERNEL_TMA)
-            step_tma<<<grid, TMA_THREADS, step_tma_smem_bytes(), ctx_.stream>>>(a);
-        else if (g->kind == MNAD_KERNEL_TMA_NARROW)
-            step_tma_narrow<<<std::min(g->ntiles, ctx_.num_sms * TMA_CTAS_PER_SM_NARROW), TMA_TZY * TMA_TX_NARROW,
-                              step_tma_narrow_smem_bytes(), ctx_.stream>>>(a);
+        // A step's launch overlaps the tail of the step before it (the kernels
+        // wait for that step themselves).  With the steps of a single run
+        // launched one by one: a shot of 1023 x 2047, 800 steps, 23.0 -> 21.3 ms
+        // (captured in a graph for one run 23.0, one by one without it 23.2).
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.stream = ctx_.stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (g->kind == MNAD_KERNEL_TMA) {
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(TMA_THREADS);
+            cfg.dynamicSmemBytes = step_tma_smem_bytes();
+            MNAD_CK(cudaLaunchKernelEx(&cfg, step_tma, a));
+        } else if (g->kind == MNAD_KERNEL_TMA_NARROW) {
+            cfg.gridDim = dim3(std::min(g->ntiles, ctx_.num_sms * TMA_CTAS_PER_SM_NARROW));
+            cfg.blockDim = dim3(TMA_TZY * TMA_TX_NARROW);
+            cfg.dynamicSmemBytes = step_tma_narrow_smem_bytes();
+            MNAD_CK(cudaLaunchKernelEx(&cfg, step_tma_narrow, a));
+        }
         else if (g->kind == MNAD_KERNEL_TMA2)
             step_tma2<<<grid, TMA_THREADS, step_tma2_smem_bytes(), ctx_.stream>>>(a);
         else

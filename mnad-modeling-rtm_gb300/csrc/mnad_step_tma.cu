@@ -117,6 +117,10 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
         if (tid == 0 && A.ntiles > 0) atomicOr(A.status, ST_TIMEOUT);
         return;
     }
+    // The launch may start while the previous step's last tiles run: its CTAs
+    // take the places of those that have left, set up their barriers and wait
+    // here until that step is complete and its stores are visible.
+    launch_dependents();
     const int cur = A.s & 1;
     // Thread 0 claims tiles from the launch's counter, one per iteration and
     // one iteration ahead (the atomic's latency stays off its path); the claim
@@ -135,6 +139,7 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
         }
         fence_mbar_init();
         *abort_flag = 0;
+        wait_for_previous_launch();
 #pragma unroll
         for (int k = 0; k < NST; ++k) {
             const int t = (int)blockIdx.x + k * (int)gridDim.x;
@@ -146,6 +151,8 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
         // copies, or the arrive of "no tile"); fill f goes to stage f % NST
         *nfills = NST;
         next_claim = first + atomicAdd(A.tile_counter, 1);
+    } else {
+        wait_for_previous_launch();
     }
     __syncthreads();
     const int tzt = tid % TMA_TZY, txt = tid / TMA_TZY;
@@ -196,7 +203,7 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
             float2 su[2], sv[2], sw[2];
             {
                 Window win;
-                win.load<FS>(&st.halo[0][0][0], c, r0);
+                win.load_run<FS>(&st.halo[0][0][0], c, r0, tzt == 0, tzt == TMA_TZY - 1);
                 mnad_update_pairs(A.coef2, win, rr, su, sv, sw);
             }
             const float4 pu = *reinterpret_cast<const float4*>(&st.pts[0][txt][tzt * Q]);
