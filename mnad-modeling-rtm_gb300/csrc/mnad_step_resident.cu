@@ -24,9 +24,9 @@
 // about equal weight; with a few hundred points the exchange, about 1 us from
 // a published cell to its use.  Time per step of one propagation, on chip /
 // the step-per-launch kernel it replaces (CUDA events, GB300):
-//   96 x 112 1.9 / 4.1 us, 201 x 201 2.1 / 4.6, 381 x 681 3.5 / 8.7,
-//   481 x 1281 5.5 / 16.9, 600 x 1200 (persistent kernel's rounding) 5.6 / 11.4,
-//   eight of 256 x 256 0.68 / 1.74 each, eight of 321 x 641 2.2 / 3.3 each.
+//   96 x 112 1.9 / 4.1 us, 201 x 201 2.1 / 4.6, 381 x 681 3.3 / 8.7,
+//   481 x 1281 5.1 / 16.9, 600 x 1200 (persistent kernel's rounding) 5.2 / 11.4,
+//   eight of 256 x 256 0.65 / 1.74 each, eight of 321 x 641 2.0 / 3.3 each.
 // Layouts that measured worse on 481 x 1281: one lane group per column with
 // idle lanes at the column ends 6.7 us; a warp marching along x with the
 // window in registers 7+; strips in a pass of their own 6.9; tasks claimed
@@ -75,6 +75,7 @@ constexpr unsigned RQ_UP = 1u << 25;          // the previous lane holds the gro
 constexpr unsigned RQ_DOWN = 1u << 26;        // the next lane holds the group below
 // order of the groups: edges on the general path, plain edges, the others alike
 constexpr int RES_CLASSES = 4;
+constexpr unsigned RES_STAGGER = 600;         // cycles between the starts of a sub-partition's warps
 static_assert(RES_RECS <= 4096, "injection slots fit the table entry");
 static_assert(RES_MAX_ROWS / 4 <= 255 && RES_MAX_COLS <= 255, "group coordinates fit the table entry");
 
@@ -250,25 +251,39 @@ __device__ __forceinline__ void load_window(Window& w, const float* f0, int fs, 
     }
     w.wz[0] = __shfl_up_sync(all, w.w[1][3], 1);
     w.wz[1] = __shfl_down_sync(all, w.w[1][2], 1);
-    if (!(flags & RQ_UP)) {
+    const bool up = flags & RQ_UP, down = flags & RQ_DOWN;
+    if (!up || !down) {
+        // one side from shared memory (with both sides missing, the other too):
+        // the two ends of a run share one set of loads
+        const int o1 = up ? Q : -1, o2 = up ? Q + 1 : -2;
+        float x[10];
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc) {
-            const float* f = f0 + (cc - 1) * RES_PITCH - 1;
-            w.u[cc][0] = f[0];
-            w.v[cc][0] = f[fs];
-            w.w[cc][0] = f[2 * fs];
+            const float* f = f0 + (cc - 1) * RES_PITCH + o1;
+            x[3 * cc] = f[0];
+            x[3 * cc + 1] = f[fs];
+            x[3 * cc + 2] = f[2 * fs];
         }
-        w.wz[0] = f0[2 * fs - 2];
-    }
-    if (!(flags & RQ_DOWN)) {
+        x[9] = f0[2 * fs + o2];
+        if (up) {
 #pragma unroll
-        for (int cc = 0; cc < 3; ++cc) {
-            const float* f = f0 + (cc - 1) * RES_PITCH + Q;
-            w.u[cc][5] = f[0];
-            w.v[cc][5] = f[fs];
-            w.w[cc][5] = f[2 * fs];
+            for (int cc = 0; cc < 3; ++cc) w.u[cc][5] = x[3 * cc], w.v[cc][5] = x[3 * cc + 1], w.w[cc][5] = x[3 * cc + 2];
+            w.wz[1] = x[9];
+        } else {
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) w.u[cc][0] = x[3 * cc], w.v[cc][0] = x[3 * cc + 1], w.w[cc][0] = x[3 * cc + 2];
+            w.wz[0] = x[9];
         }
-        w.wz[1] = f0[2 * fs + Q + 1];
+        if (!up && !down) {
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) {
+                const float* f = f0 + (cc - 1) * RES_PITCH + Q;
+                w.u[cc][5] = f[0];
+                w.v[cc][5] = f[fs];
+                w.w[cc][5] = f[2 * fs];
+            }
+            w.wz[1] = f0[2 * fs + Q + 1];
+        }
     }
 }
 
@@ -1043,6 +1058,18 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
             S.inj = C.L.inj + (s & 1) * 4 * RES_RECS;
             S.out = C.out && s + 1 < C.s_end ? C.out + ((s + 1) & 1) * C.plane : nullptr;
             const int ntask = C.ntask, warps = nwork >> 5;
+            if constexpr (!SMALL) {
+                // The warps of an SM sub-partition start one after the other.
+                // Released together by the barrier they load together and then
+                // compute together, and each pipe idles through the other's
+                // phase; staggered by a third of a task they overlap, and the
+                // first four warps, which hold the edges, publish earlier.
+                // 600 cycles: 481 x 1281 5.45 -> 5.10 us a step, 381 x 681 3.50
+                // -> 3.30, 600 x 1200 5.69 -> 5.20 (300: 5.20, 3.38, 5.31; 900:
+                // 5.25, 3.21, 5.28; turns passed by named barriers: 5.69, 3.45, 5.74).
+                const unsigned t0 = clock(), wait = (tid >> 7) * RES_STAGGER;
+                while ((unsigned)clock() - t0 < wait) {}
+            }
             float peak = 0.0f;                                // largest |d2u| of a snapshot
             for (int k = tid >> 5; k < ntask; k += warps) {
                 if constexpr (SMALL) {
