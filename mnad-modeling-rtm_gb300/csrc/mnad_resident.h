@@ -48,7 +48,8 @@ struct ResLayout {
     int r, xm, ztm, zbm, xk, ztk, zbk, inj, qtab, qinj, halo, recs, misc, total;
 };
 
-MNAD_HD ResLayout res_layout(const ResPatch& p, int nz, int nx, int d)
+// small: the patch goes point by point (a table entry per point instead of per group)
+MNAD_HD ResLayout res_layout(const ResPatch& p, int nz, int nx, int d, bool small = false)
 {
     ResLayout L;
     L.fs = (p.ni + 4) * RES_PITCH;
@@ -72,7 +73,7 @@ MNAD_HD ResLayout res_layout(const ResPatch& p, int nz, int nx, int d)
     L.ztk = o;    o += 3 * p.ni * L.zt;
     L.zbk = o;    o += 3 * p.ni * L.zb;
     L.inj = o;    o += 2 * 4 * RES_RECS;
-    L.qtab = o;   o += 4 * L.nquads;
+    L.qtab = o;   o += (small ? 16 : 4) * L.nquads;
     L.qinj = o;   o += L.nquads;
     o = (o + 3) & ~3;
     L.halo = o;   o += 2 * L.nhalo;
@@ -187,12 +188,14 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
         cut(hi, &p.patches, &p.band_first);
         p.cost = hi;
         for (const ResPatch& q : p.patches) {
-            p.smem = std::max(p.smem, (size_t)res_layout(q, nz, nx, d).total * 4);
             p.slots = std::max(p.slots, res_slots(q.nj, q.ni));
             p.small &= q.nj * q.ni <= RES_SMALL;
         }
         int tasks = 0;
-        for (const ResPatch& q : p.patches) tasks = std::max(tasks, res_tasks(q.nj, q.ni, p.small));
+        for (const ResPatch& q : p.patches) {
+            tasks = std::max(tasks, res_tasks(q.nj, q.ni, p.small));
+            p.smem = std::max(p.smem, (size_t)res_layout(q, nz, nx, d, p.small).total * 4);
+        }
         // one warp does the exchange, two where the compute warps go round as
         // often without the second
         const int warps = (p.small ? RES_POINT_THREADS : RES_THREADS) / 32;

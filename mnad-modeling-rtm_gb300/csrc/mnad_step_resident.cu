@@ -24,7 +24,7 @@
 // about equal weight; with a few hundred points the exchange, about 1 us from
 // a published cell to its use.  Time per step of one propagation, on chip /
 // the step-per-launch kernel it replaces (CUDA events, GB300):
-//   96 x 112 1.9 / 4.1 us, 201 x 201 2.1 / 4.6, 381 x 681 3.3 / 8.7,
+//   96 x 112 1.7 / 4.1 us, 201 x 201 2.1 / 4.6, 381 x 681 3.3 / 8.7,
 //   481 x 1281 5.1 / 16.9, 600 x 1200 (persistent kernel's rounding) 5.2 / 11.4,
 //   eight of 256 x 256 0.65 / 1.74 each, eight of 321 x 641 2.0 / 3.3 each.
 // Layouts that measured worse on 481 x 1281: one lane group per column with
@@ -57,11 +57,12 @@ namespace {
 using namespace tile;
 
 constexpr int Q = TMA_PZ;
-// Table entry of a group (offsets in floats):
+// Table entry of a group, or of a point of a small patch (offsets in floats):
 //   x: its place in a staged field | flags
 //   y: its place in r | in the x strips' arrays << 16
 //   z: its place in the top strip's arrays | in the bottom strip's << 16
-//   w: group row (4-row units) | column << 8 | injection slot << 16
+//   z of a point: its place in its z strip's arrays | its publication slot << 16
+//   w: group row (4-row units; a point's row) | column << 8 | injection slot << 16
 constexpr unsigned RQ_EDGE = 1u << 16;        // holds cells that other patches need
 constexpr unsigned RQ_X = 1u << 17;           // in an x strip
 constexpr unsigned RQ_RIGHT = 1u << 18;       // in the right one
@@ -73,6 +74,7 @@ constexpr unsigned RQ_PAST = 1u << 23;        // rows past nz
 constexpr unsigned RQ_GENERAL = 1u << 24;     // any of the seven above
 constexpr unsigned RQ_UP = 1u << 25;          // the previous lane holds the group above
 constexpr unsigned RQ_DOWN = 1u << 26;        // the next lane holds the group below
+constexpr unsigned RQ_IMAGE = 1u << 27;       // in the image region (points)
 // order of the groups: edges on the general path, plain edges, the others alike
 constexpr int RES_CLASSES = 4;
 constexpr unsigned RES_STAGGER = 600;         // cycles between the starts of a sub-partition's warps
@@ -112,7 +114,7 @@ struct PatchCtx {
     int nhalo, nrec;                        // cells polled; receivers in the table
     int single;                             // the launch runs one step
     int ntask;                              // warp tasks of a step
-    float inv_nj;
+    int vsx, vst, vsb;                      // strides of the strips' variables
     int s_end;                              // the launch's last step + 1 for this propagation
     uint4* words;                           // published cells of the propagation [parity][patch][slot]
     uint4* out;                             // this patch's, of parity 0 (null: nobody needs them)
@@ -527,18 +529,19 @@ __device__ __forceinline__ float strip_point(const float* c, float ih, float fd,
     return m1;
 }
 
-// Row lr, column c of the patch: the new U, V, W into S.nxt, and the cell out if
-// other patches need it.
+// One point: the new U, V, W into S.nxt, and the cell out if other patches need
+// it.  Where everything of the point lies is in its table entry, built once: worked
+// out in every step it cost more instructions than the stencil (197 integer to
+// 131 FP32 per point; a step of 201 x 201 2.26 -> 2.16 us, of 300 x 300 2.87 -> 2.70).
 template <bool POINT_ORDER>
 __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, const PatchCtx& C, const StepCtx& S,
-                                           float* sm, int lr, int c, float& peak)
+                                           float* sm, const uint4 e, float& peak)
 {
     constexpr int X = RES_PITCH;
-    const int fs = C.L.fs, nj = C.nj, o = (c + 2) * X + 4 + lr;
-    const int j = C.j0 + lr, i = C.i0 + c, d = P.d, nz = P.nz, nx = P.nx;
+    const int fs = C.L.fs, o = e.x & 0xffff;
     const float *u = S.cur + o, *v = u + fs, *w = v + fs;
     float* n = S.nxt + o;
-    const float r = sm[C.L.r + c * nj + lr];
+    const float r = sm[C.L.r + (e.y & 0xffff)];
     Hood h;
     h.u00 = u[0]; h.uzm = u[-1]; h.uzp = u[1]; h.uxm = u[-X]; h.uxp = u[X];
     h.umm = u[-X - 1]; h.upm = u[-X + 1]; h.ump = u[X - 1]; h.upp = u[X + 1];
@@ -548,13 +551,12 @@ __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, c
     h.wmm = w[-X - 1]; h.wpm = w[-X + 1]; h.wmp = w[X - 1]; h.wpp = w[X + 1]; h.wzm2 = w[-2]; h.wzp2 = w[2];
     float s[3];
     update_point<POINT_ORDER>(K, r, h, s);
-    const bool in_x = i < d || i >= nx - d, in_z = (j < d || j >= nz - d) && j < nz;
-    const int dj = C.src_row - j, di = C.src_col - i;     // to the source
-    if (in_x || in_z) {
+    if (e.x & (RQ_X | RQ_TOP | RQ_BOTTOM)) {
         // the CPML sees U before this step's injection (fwd_PDE_exact_MNAD.m:95-111)
         float u0 = h.u00, uxm = h.uxm, uxp = h.uxp, uzm = h.uzm, uzp = h.uzp;
-        if (abs(dj) + abs(di) <= 1) {
+        if (e.x & RQ_SOURCE) {
             const float amp = P.src_amp[S.tt - 1];
+            const int dj = C.src_row - C.j0 - (int)(e.w & 0xff), di = C.src_col - C.i0 - (int)((e.w >> 8) & 0xff);
             if (dj == 0 && di == 0) u0 -= amp;
             else if (di == -1) uxm -= amp;
             else if (di == 1) uxp -= amp;
@@ -562,9 +564,9 @@ __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, c
             else uzp -= amp;
         }
         float cp[3] = {0.0f, 0.0f, 0.0f};
-        if (in_x) {
-            const bool low = i < d;
-            const int at = (low ? c : C.L.xleft + (i - max(C.i0, nx - d))) * nj + lr, vs = C.L.xcols * nj;
+        if (e.x & RQ_X) {
+            const bool low = !(e.x & RQ_RIGHT);
+            const int at = e.y >> 16, vs = C.vsx;
             const float* kc = sm + C.L.xk + at;
             const float k[3] = {kc[0], kc[vs], kc[2 * vs]};
             float* m = sm + C.L.xm + at;
@@ -572,9 +574,9 @@ __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, c
             cp[1] += strip_point(k, C.ihx, h.vxm, h.v00, h.vxp, low, m + 3 * vs, vs);
             cp[2] += strip_point(k, C.ihx, h.wxm, h.w00, h.wxp, low, m + 6 * vs, vs);
         }
-        if (in_z) {
-            const bool low = j < d;
-            const int rows = low ? C.L.zt : C.L.zb, at = c * rows + (low ? lr : j - C.L.zb_first), vs = C.ni * rows;
+        if (e.x & (RQ_TOP | RQ_BOTTOM)) {
+            const bool low = e.x & RQ_TOP;
+            const int at = e.z & 0xffff, vs = low ? C.vst : C.vsb;
             const float* kc = sm + (low ? C.L.ztk : C.L.zbk) + at;
             const float k[3] = {kc[0], kc[vs], kc[2 * vs]};
             float* m = sm + (low ? C.L.ztm : C.L.zbm) + at;
@@ -592,29 +594,26 @@ __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, c
     float ow = h.w00 + ((h.w00 - n[2 * fs]) + s[2]);
     if (P.mode == MODE_FWD) {
         // the next step's injection (fwd_PDE_exact_MNAD.m:111): stored U holds it
-        if (dj == 0 && di == 0 && S.tt < P.nt) ou += P.src_amp[S.tt];
-    } else if (S.tt < P.nt) {
+        if ((e.x & RQ_SOURCE) && S.tt < P.nt && C.j0 + (int)(e.w & 0xff) == C.src_row &&
+            C.i0 + (int)((e.w >> 8) & 0xff) == C.src_col)
+            ou += P.src_amp[S.tt];
+    } else if ((e.x & RQ_INJECT) && S.tt < P.nt) {
         // Born_adj_MNAD.m:109-111: the residual of step tt+1 enters U after the update
-        const unsigned slot = reinterpret_cast<const unsigned*>(sm + C.L.qinj)[c * (nj / Q) + lr / Q];
-        if (slot != 0) {
-            float inj = 0.0f;
-            if (C.inj_scan) inj = adjoint_injection(P, S.tt, (j / TMA_TZ + (i / TMA_TX) * P.ntz) * TMA_TX + i % TMA_TX,
-                                                    (size_t)(i + HX) * P.ld + (j + HZ));
-            else inj = sm[S.inj + (slot & 0xffff) * Q + lr % Q];
-            ou -= inj;
-        }
+        const int j = C.j0 + (int)(e.w & 0xff), i = C.i0 + (int)((e.w >> 8) & 0xff);
+        float inj = 0.0f;
+        if (C.inj_scan) inj = adjoint_injection(P, S.tt, (j / TMA_TZ + (i / TMA_TX) * P.ntz) * TMA_TX + i % TMA_TX,
+                                                (size_t)(i + HX) * P.ld + (j + HZ));
+        else inj = sm[S.inj + (e.w >> 16)];
+        ou -= inj;
     }
-    if (j >= nz) ou = ov = ow = 0.0f;                     // rows past nz are the zero halo
+    if (e.x & RQ_PAST) ou = ov = ow = 0.0f;               // rows past nz are the zero halo
     n[0] = ou;
     n[fs] = ov;
     n[2 * fs] = ow;
-    if (S.out) {
-        const int slot = res_slot(nj, C.ni, lr, c);
-        if (slot >= 0) publish(S.out + slot, ou, ov, ow, S.tag);
-    }
-    if (S.snap_step && i >= d && i < nx - d && j >= d && j < nz - d) {
-        const int niz = nz - 2 * d;
-        const size_t nint = (size_t)niz * (nx - 2 * d), q = (size_t)(j - d) + (size_t)(i - d) * niz;
+    if (S.out && (e.x & RQ_EDGE)) publish(S.out + (e.z >> 16), ou, ov, ow, S.tag);
+    if (S.snap_step && (e.x & RQ_IMAGE)) {
+        const int d = P.d, j = C.j0 + (int)(e.w & 0xff), i = C.i0 + (int)((e.w >> 8) & 0xff), niz = P.nz - 2 * d;
+        const size_t nint = (size_t)niz * (P.nx - 2 * d), q = (size_t)(j - d) + (size_t)(i - d) * niz;
         if (P.mode == MODE_FWD) {
             // fwd_PDE_exact_MNAD.m:128-141; nU - 2U + pU = su
             float d2u = s[0];
@@ -817,7 +816,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     const int sa = max(A.s0, max(P.s_begin, P.s_off)), sb = min(A.s1, min(P.s_end, P.s_off + P.nt));
     if (sa >= sb) return;
     const int nz = P.nz, nx = P.nx, d = P.d, ld = P.ld;
-    const ResLayout L = res_layout(patch, nz, nx, d);
+    const ResLayout L = res_layout(patch, nz, nx, d, SMALL);
     const int j0 = patch.j0, nj = patch.nj, i0 = patch.i0, ni = patch.ni, nqz = nj / Q;
     uint4* qtab = reinterpret_cast<uint4*>(sm + L.qtab);
     unsigned* qinj = reinterpret_cast<unsigned*>(sm + L.qinj);
@@ -950,6 +949,29 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     // run of groups, the counts per warp and class give every warp its places
     const int zs = P.src >= 0 ? P.src % ld - HZ : -8, xsrc = P.src >= 0 ? P.src / ld - HX : -8;
     const int run = (L.nquads + nwarps * 32 - 1) / (nwarps * 32) * 32, q0 = warp * run, q1 = min(q0 + run, L.nquads);
+    if constexpr (SMALL)
+        for (int n = tid; n < nj * ni; n += nthr) {
+            const int c = n / nj, lr = n - c * nj, j = j0 + lr, i = i0 + c;
+            const unsigned inj = qinj[c * nqz + lr / Q];
+            unsigned fl = inj & RQ_INJECT;
+            if (i < d) fl |= RQ_X;
+            else if (i >= nx - d) fl |= RQ_X | RQ_RIGHT;
+            if (j < d) fl |= RQ_TOP;
+            else if (j >= nz - d && j < nz) fl |= RQ_BOTTOM;
+            if (P.src >= 0 && abs(i - xsrc) + abs(j - zs) <= 1) fl |= RQ_SOURCE;
+            if (j >= nz) fl |= RQ_PAST;
+            if (i >= d && i < nx - d && j >= d && j < nz - d) fl |= RQ_IMAGE;
+            const int slot = A.npatch > 1 ? res_slot(nj, ni, lr, c) : -1;
+            if (slot >= 0) fl |= RQ_EDGE;
+            const int xc = i < d ? c : L.xleft + (i - max(i0, nx - d));
+            uint4 e;
+            e.x = (unsigned)((c + 2) * RES_PITCH + 4 + lr) | fl;
+            e.y = (unsigned)n | (fl & RQ_X ? (unsigned)(xc * nj + lr) << 16 : 0u);
+            e.z = (fl & RQ_TOP ? (unsigned)(c * L.zt + lr) : fl & RQ_BOTTOM ? (unsigned)(c * L.zb + j - L.zb_first) : 0u) |
+                  (slot >= 0 ? (unsigned)slot << 16 : 0u);
+            e.w = (unsigned)lr | (unsigned)c << 8 | ((inj & 0xffff) * Q + lr % Q) << 16;
+            qtab[n] = e;
+        }
     for (int pass = 0; pass < 2 && !SMALL; ++pass) {
         int at[RES_CLASSES] = {0, 0, 0, 0};
         if (pass == 1) {
@@ -1013,7 +1035,9 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
         C.nhalo = nhalo;
         C.nrec = nrec;
         C.single = sb - sa == 1;
-        C.inv_nj = 1.0f / (float)nj;
+        C.vsx = L.xcols * nj;
+        C.vst = ni * L.zt;
+        C.vsb = ni * L.zb;
         C.ntask = res_tasks(nj, ni, SMALL);
         C.s_end = sb;
         C.plane = (size_t)A.npatch * A.slots;
@@ -1073,8 +1097,8 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
             float peak = 0.0f;                                // largest |d2u| of a snapshot
             for (int k = tid >> 5; k < ntask; k += warps) {
                 if constexpr (SMALL) {
-                    const int n = 32 * k + lane, c = (int)(((float)n + 0.5f) * C.inv_nj);
-                    if (c < C.ni) point_step<POINT_ORDER>(A.coef2, P, C, S, sm, n - c * C.nj, c, peak);
+                    const int n = 32 * k + lane;
+                    if (n < C.nj * C.ni) point_step<POINT_ORDER>(A.coef2, P, C, S, sm, qtab[n], peak);
                 } else {
                     // the general path if one of the warp's groups needs it
                     const int nquads = C.L.nquads;
