@@ -316,6 +316,27 @@ __device__ __forceinline__ float snap_decode(const void* base, int codec, size_t
     return static_cast<const float*>(base)[i];
 }
 
+// Four neighbouring samples: one branch, four loads in flight.
+__device__ __forceinline__ void snap_decode4(const void* base, int codec, size_t i, float scale, float* out)
+{
+    if (codec == CODEC_BF16) {
+        __nv_bfloat16 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = static_cast<const __nv_bfloat16*>(base)[i + k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k] = __bfloat162float(x[k]);
+    } else if (codec == CODEC_F16) {
+        __half x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = static_cast<const __half*>(base)[i + k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k] = __half2float(x[k]) * scale;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k] = static_cast<const float*>(base)[i + k];
+    }
+}
+
 // Power-of-two scale s of an FP16 snapshot, chosen from its largest |x| = mx so
 // that mx/s < 2^14 (no saturation; the scale multiply is exact), and 1/s.
 // Arrays whose maximum is below 2^-100 keep s = 2^-114, so 1/s stays finite.
@@ -356,6 +377,19 @@ __device__ __forceinline__ void accumulate_product(double* acc, float a, float b
     const float p = __fmul_rn(a, b);
     if (p == 0.0f) return;
     *acc += widen_f32(p);
+}
+
+// accumulate_product of four neighbouring accumulators, from their products:
+// all loads before the first store (one after the other each load waits for the
+// store before it, four trips to L2 per group).
+__device__ __forceinline__ void accumulate4(double* acc, const float* p)
+{
+    double a[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = p[k] != 0.0f ? acc[k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (p[k] != 0.0f) acc[k] = a[k] + widen_f32(p[k]);
 }
 
 }  // namespace mnad

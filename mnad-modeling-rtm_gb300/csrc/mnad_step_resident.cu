@@ -136,53 +136,94 @@ struct StepCtx {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// Snapshot and illumination (forward) or image (adjoint) of a group's points
-// inside the image region at a snapshot step.
+// Snapshot and illumination of a group's points inside the image region at a
+// forward's snapshot step.
 __device__ __forceinline__ void snapshot(const PropDesc& P, const StepCtx& S, int j, int i, const float2* su,
-                                         const float4& uc4, const float4& pu4, const float* ou, float& peak)
+                                         const float4& uc4, const float4& pu4, float& peak)
 {
     const int d = P.d, nz = P.nz, nx = P.nx, niz = nz - 2 * d;
     if (!(i >= d && i < nx - d)) return;
     const size_t nint = (size_t)niz * (nx - 2 * d);
     const long long q0 = (long long)(j - d) + (long long)(i - d) * niz;
-    if (P.mode == MODE_FWD) {
-        const float sus[Q] = {su[0].x, su[0].y, su[1].x, su[1].y};
-        const float pus[Q] = {pu4.x, pu4.y, pu4.z, pu4.w};
-        const float ucs[Q] = {uc4.x, uc4.y, uc4.z, uc4.w};
-        const int slot = P.snap_stage ? 0 : S.tq - 1 - P.snap_col0;
-        const bool keep = (P.snap_flags & SNAP_WRITE) && slot >= 0 && slot < P.snap_cols;
+    const float sus[Q] = {su[0].x, su[0].y, su[1].x, su[1].y};
+    const float pus[Q] = {pu4.x, pu4.y, pu4.z, pu4.w};
+    const float ucs[Q] = {uc4.x, uc4.y, uc4.z, uc4.w};
+    const int slot = P.snap_stage ? 0 : S.tq - 1 - P.snap_col0;
+    const bool keep = (P.snap_flags & SNAP_WRITE) && slot >= 0 && slot < P.snap_cols;
+    float sq[Q] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int k = 0; k < Q; ++k) {
-            const int jk = j + k;
-            if (!(jk >= d && jk < nz - d)) continue;
-            // fwd_PDE_exact_MNAD.m:128-141; nU - 2U + pU = su
-            float d2u = sus[k];
-            if (S.tt == 1) d2u = fmaf(2.0f, ucs[k], sus[k] - pus[k]);
-            else if (S.tt == 2) d2u = sus[k] - pus[k];
-            d2u *= P.inv_dt2;
-            const size_t q = (size_t)(q0 + k);
-            if (keep) {
-                const size_t at = (size_t)slot * nint + q;
-                if (P.codec == CODEC_BF16) static_cast<__nv_bfloat16*>(P.snap)[at] = __float2bfloat16_rn(d2u);
-                else static_cast<float*>(P.snap)[at] = d2u;
-                peak = fmaxf(peak, fabsf(d2u));
-            }
-            if (P.snap_flags & SNAP_ILLUM) accumulate_product(&P.illum[q], d2u, d2u);
+    for (int k = 0; k < Q; ++k) {
+        const int jk = j + k;
+        if (!(jk >= d && jk < nz - d)) continue;
+        // fwd_PDE_exact_MNAD.m:128-141; nU - 2U + pU = su
+        float d2u = sus[k];
+        if (S.tt == 1) d2u = fmaf(2.0f, ucs[k], sus[k] - pus[k]);
+        else if (S.tt == 2) d2u = sus[k] - pus[k];
+        d2u *= P.inv_dt2;
+        if (keep) {
+            const size_t at = (size_t)slot * nint + (size_t)(q0 + k);
+            if (P.codec == CODEC_BF16) static_cast<__nv_bfloat16*>(P.snap)[at] = __float2bfloat16_rn(d2u);
+            else static_cast<float*>(P.snap)[at] = d2u;
+            peak = fmaxf(peak, fabsf(d2u));
         }
-    } else {
-        // Born_adj_MNAD.m:127-134
-        const int col = (P.pairing == PAIR_REFERENCE ? P.ncols : P.nsnap) - (P.img_steps - S.tq);
-        if (col < 1 || col > P.nsnap || col - 1 < P.snap_col0 || col - 1 - P.snap_col0 >= P.snap_cols) return;
-        const float sc = P.codec == CODEC_F16 ? P.snap_scale[col - 1] : 1.0f;
-        const size_t at = (size_t)(col - 1 - P.snap_col0) * nint;
-#pragma unroll
-        for (int k = 0; k < Q; ++k) {
-            const int jk = j + k;
-            if (!(jk >= d && jk < nz - d)) continue;
-            const size_t q = (size_t)(q0 + k);
-            accumulate_product(&P.image[q], snap_decode(P.snap, P.codec, at + q, sc), ou[k]);
-        }
+        sq[k] = __fmul_rn(d2u, d2u);
     }
+    if (P.snap_flags & SNAP_ILLUM) accumulate4(P.illum + q0, sq);
+}
+
+// Born_adj_MNAD.m:127-134: the snapshot column that an adjoint's step tt = tq T
+// images with, from 0; -1 for none.
+__device__ __forceinline__ int image_column(const PropDesc& P, int tq)
+{
+    const int col = (P.pairing == PAIR_REFERENCE ? P.ncols : P.nsnap) - (P.img_steps - tq) - 1;
+    return col >= 0 && col < P.nsnap && col >= P.snap_col0 && col - P.snap_col0 < P.snap_cols ? col : -1;
+}
+
+// Adds the patch's image terms: U of the level at `level` (staged), snapshot
+// column col.  Done by the warps of the step after the imaging step, as they run
+// out of groups: along the columns, G at a time, all loads before the first
+// store.  Inside the group's own update the loads were strided and their
+// latency stood before the step's barrier (an adjoint of 481 x 1281 that images
+// at every step 10.7 -> 7.7 us a step, at every eighth 6.05 -> 5.41).
+template <int G, int CODEC>
+__device__ __forceinline__ void add_image_as(const PropDesc& P, const PatchCtx& C, const float* level, int col, int warp, int warps)
+{
+    const int d = P.d, niz = P.nz - 2 * d, lane = threadIdx.x & 31;
+    const size_t nint = (size_t)niz * (P.nx - 2 * d);
+    const int ja = max(C.j0, d), n = min(C.j0 + C.nj, P.nz - d) - ja, ia = max(C.i0, d), m = min(C.i0 + C.ni, P.nx - d) - ia;
+    const size_t q0 = (size_t)(ja - d) + (size_t)(ia - d) * niz, at = (size_t)(col - P.snap_col0) * nint;
+    const float sc = CODEC == CODEC_F16 ? P.snap_scale[col] : 1.0f;
+    const float* u0 = level + (ia - C.i0 + 2) * RES_PITCH + 4 + (ja - C.j0);
+    constexpr int R = RES_MAX_ROWS / 32;
+    const void* snap = P.snap;
+    double* image = P.image;
+    for (int c0 = warp; c0 < m; c0 += G * warps) {
+        float p[G][R];
+        double a[G][R];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int c = c0 + g * warps, row = lane + 32 * r;
+                const bool in = c < m && row < n;
+                const size_t q = q0 + (size_t)c * niz + row;
+                p[g][r] = in ? __fmul_rn(snap_decode(snap, CODEC, at + q, sc), u0[c * RES_PITCH + row]) : 0.0f;
+                a[g][r] = in ? image[q] : 0.0;
+            }
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (p[g][r] != 0.0f)                      // as accumulate_product
+                    image[q0 + (size_t)(c0 + g * warps) * niz + lane + 32 * r] = a[g][r] + widen_f32(p[g][r]);
+    }
+}
+template <int G>
+__device__ __forceinline__ void add_image(const PropDesc& P, const PatchCtx& C, const float* level, int col, int warp, int warps)
+{
+    if (P.codec == CODEC_BF16) add_image_as<G, CODEC_BF16>(P, C, level, col, warp, warps);
+    else if (P.codec == CODEC_F16) add_image_as<G, CODEC_F16>(P, C, level, col, warp, warps);
+    else add_image_as<G, CODEC_F32>(P, C, level, col, warp, warps);
 }
 
 // nF = F + ((F - pF) + sF) of a group.
@@ -426,7 +467,7 @@ __device__ __forceinline__ void group_step(const Coefs2& K, const PropDesc& P, c
             }
         }
     }
-    if (S.snap_step) snapshot(P, S, C.j0 + zq * Q, C.i0 + c, s[0], uc, pu, ou, peak);
+    if (S.snap_step) snapshot(P, S, C.j0 + zq * Q, C.i0 + c, s[0], uc, pu, peak);
 }
 
 // mnad_update_pairs at one point.
@@ -614,29 +655,19 @@ __device__ __forceinline__ void point_step(const Coefs2& K, const PropDesc& P, c
     if (S.snap_step && (e.x & RQ_IMAGE)) {
         const int d = P.d, j = C.j0 + (int)(e.w & 0xff), i = C.i0 + (int)((e.w >> 8) & 0xff), niz = P.nz - 2 * d;
         const size_t nint = (size_t)niz * (P.nx - 2 * d), q = (size_t)(j - d) + (size_t)(i - d) * niz;
-        if (P.mode == MODE_FWD) {
-            // fwd_PDE_exact_MNAD.m:128-141; nU - 2U + pU = su
-            float d2u = s[0];
-            if (S.tt == 1) d2u = fmaf(2.0f, h.u00, s[0] - pu);
-            else if (S.tt == 2) d2u = s[0] - pu;
-            d2u *= P.inv_dt2;
-            const int slot = P.snap_stage ? 0 : S.tq - 1 - P.snap_col0;
-            if ((P.snap_flags & SNAP_WRITE) && slot >= 0 && slot < P.snap_cols) {
-                const size_t at = (size_t)slot * nint + q;
-                if (P.codec == CODEC_BF16) static_cast<__nv_bfloat16*>(P.snap)[at] = __float2bfloat16_rn(d2u);
-                else static_cast<float*>(P.snap)[at] = d2u;
-                peak = fmaxf(peak, fabsf(d2u));
-            }
-            if (P.snap_flags & SNAP_ILLUM) accumulate_product(&P.illum[q], d2u, d2u);
-        } else {
-            // Born_adj_MNAD.m:127-134
-            const int col = (P.pairing == PAIR_REFERENCE ? P.ncols : P.nsnap) - (P.img_steps - S.tq);
-            if (col >= 1 && col <= P.nsnap && col - 1 >= P.snap_col0 && col - 1 - P.snap_col0 < P.snap_cols) {
-                const float sc = P.codec == CODEC_F16 ? P.snap_scale[col - 1] : 1.0f;
-                accumulate_product(&P.image[q], snap_decode(P.snap, P.codec, (size_t)(col - 1 - P.snap_col0) * nint + q, sc),
-                                   ou);
-            }
+        // fwd_PDE_exact_MNAD.m:128-141; nU - 2U + pU = su
+        float d2u = s[0];
+        if (S.tt == 1) d2u = fmaf(2.0f, h.u00, s[0] - pu);
+        else if (S.tt == 2) d2u = s[0] - pu;
+        d2u *= P.inv_dt2;
+        const int slot = P.snap_stage ? 0 : S.tq - 1 - P.snap_col0;
+        if ((P.snap_flags & SNAP_WRITE) && slot >= 0 && slot < P.snap_cols) {
+            const size_t at = (size_t)slot * nint + q;
+            if (P.codec == CODEC_BF16) static_cast<__nv_bfloat16*>(P.snap)[at] = __float2bfloat16_rn(d2u);
+            else static_cast<float*>(P.snap)[at] = d2u;
+            peak = fmaxf(peak, fabsf(d2u));
         }
+        if (P.snap_flags & SNAP_ILLUM) accumulate_product(&P.illum[q], d2u, d2u);
     }
 }
 
@@ -824,7 +855,8 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     int2* recs = reinterpret_cast<int2*>(sm + L.recs);
     int* misc = reinterpret_cast<int*>(sm + L.misc);     // 0: halo cells, 1: receivers, 2: injection slots,
                                                          // 3: duplicate receivers, 4, 5: largest |d2u| of a
-                                                         // snapshot by step parity, 6: of all patches, 16..: groups per warp and class
+                                                         // snapshot by step parity, 6: of all patches, 8, 9: the
+                                                         // step's image column by step parity, 16..: groups per warp and class
     // ---- load the patch: a warp per staged column, a few columns in flight ----
     const int nwarps = nthr >> 5;
     {
@@ -1025,6 +1057,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
         __syncthreads();
     }
     if (tid == 0) {
+        misc[8] = misc[9] = -1;                           // no step before the first
         C.L = L;
         C.j0 = j0; C.nj = nj; C.i0 = i0; C.ni = ni;
         C.ihx = 1.0f / P.dx;
@@ -1058,6 +1091,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     __syncthreads();
     // ---- the steps ------------------------------------------------------------
     int staged = 0;                                       // number of the snapshot that is not encoded yet
+    const bool staging = P.snap_stage != 0;
     for (int s = sa; s < C.s_end; ++s) {
         // words of the descriptor and the patch are read again in every step
         // (kept in registers they spill)
@@ -1078,7 +1112,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
         const int comm = A.comm, nwork = blockDim.x - comm;   // compute threads; the last warps do the exchange
         if (tid < nwork) {
             S.tq = (int)(((float)S.tt + 0.5f) * P.invT);
-            S.snap_step = P.T > 0 && S.tt - S.tq * P.T == 0;
+            S.snap_step = fwd && P.T > 0 && S.tt - S.tq * P.T == 0;
             S.inj = C.L.inj + (s & 1) * 4 * RES_RECS;
             S.out = C.out && s + 1 < C.s_end ? C.out + ((s + 1) & 1) * C.plane : nullptr;
             const int ntask = C.ntask, warps = nwork >> 5;
@@ -1114,6 +1148,9 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
                 const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(peak));
                 if (lane == 0 && m > 0) atomicMax(reinterpret_cast<unsigned*>(sm + C.L.misc) + 4 + (s & 1), m);
             }
+            // the image terms of the step before, whose U is the current level now
+            const int image = reinterpret_cast<const int*>(sm + C.L.misc)[8 + ((s + 1) & 1)];
+            if (image >= 0) add_image<SMALL ? 1 : 4>(P, C, S.cur, image, tid >> 5, warps);
         } else {
             // forward receivers (fwd_PDE_exact_MNAD.m:119-123): U after this
             // step's injection, before its update
@@ -1126,6 +1163,11 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
                 if (P.dataw) P.dataw[at] = S.cur[2 * fs + off];
             };
             const int ct = tid - nwork;
+            if (ct == 0) {
+                const int tq = (int)(((float)S.tt + 0.5f) * P.invT);
+                reinterpret_cast<int*>(sm + C.L.misc)[8 + (s & 1)] =
+                    !fwd && P.T > 0 && S.tt - tq * P.T == 0 ? image_column(P, tq) : -1;
+            }
             if (fwd && !C.inj_scan) {
                 for (int k = ct; k < C.nrec; k += comm) record(recs[k].x, recs[k].y);
             } else if (fwd) {
@@ -1155,7 +1197,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
             if (tid == 0) atomicOr(A.status, ST_TIMEOUT);
             return;
         }
-        if (P.snap_stage) {
+        if (staging) {
             // the patch's maximum goes out; the snapshot is encoded where all
             // patches' are due: before the next one, or after the last step
             const int tq = (int)(((float)S.tt + 0.5f) * P.invT);
@@ -1178,6 +1220,9 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     }
     // ---- write the state back (the layout from shared memory) --------------------
     asm volatile("" ::: "memory");
+    const int image = reinterpret_cast<const int*>(sm + C.L.misc)[8 + ((C.s_end + 1) & 1)];
+    if (image >= 0)
+        add_image<SMALL ? 1 : 4>(P, C, sm + (C.s_end & 1) * 3 * C.L.fs, image, threadIdx.x >> 5, blockDim.x >> 5);
     {
         const ResPatch p{C.j0, C.nj, C.i0, C.ni};
         const int s0 = max(A.s0, max(P.s_begin, P.s_off)), nqe = p.nj / Q, nw = blockDim.x >> 5;

@@ -244,8 +244,10 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
                         }
                     }
                     if (P.snap_flags & SNAP_ILLUM) {
+                        float sq[Q];
 #pragma unroll
-                        for (int k = 0; k < Q; ++k) accumulate_product(&P.illum[q0 + k], d2u[k], d2u[k]);
+                        for (int k = 0; k < Q; ++k) sq[k] = __fmul_rn(d2u[k], d2u[k]);
+                        accumulate4(P.illum + q0, sq);
                     }
                 } else {
                     // Born_adj_MNAD.m:127-134
@@ -254,11 +256,11 @@ __device__ __forceinline__ void step_tma_body(const StepArgs& A)
                         const float sc = P.codec == CODEC_F16 ? P.snap_scale[col - 1] : 1.0f;
                         const size_t o = (size_t)(col - 1 - P.snap_col0) * nint + q0;
                         const float ou[Q] = {nu01.x, nu01.y, nu23.x, nu23.y};
+                        float us[Q];
+                        snap_decode4(P.snap, P.codec, o, sc, us);
 #pragma unroll
-                        for (int k = 0; k < Q; ++k) {
-                            const float us = snap_decode(P.snap, P.codec, o + k, sc);
-                            accumulate_product(&P.image[q0 + k], us, ou[k]);
-                        }
+                        for (int k = 0; k < Q; ++k) us[k] = __fmul_rn(us[k], ou[k]);
+                        accumulate4(P.image + q0, us);
                     }
                 }
             }
