@@ -124,22 +124,16 @@ void upload(Context& ctx, void* dst, const void* src, size_t bytes)
     ctx.h2d += bytes;
 }
 
-// Makes the pages of a result buffer present before the device writes into it.
-// Fresh host memory (an untouched allocation) is otherwise faulted in by the
-// copy, page by page from the device: 12 ms for a 15 MB record, against 4 ms of
-// CPU work that mostly overlaps the kernels still running (a shot of 481 x 1281,
-// 1600 steps, into a new array: 22 -> 10 ms).  No byte changes its value.
-static void touch_pages(void* dst, size_t bytes)
+void touch_pages(void* dst, size_t bytes)
 {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    if (bytes < (1u << 18)) return;
+    if (bytes < TOUCH_MIN || bytes > TOUCH_MAX) return;
     volatile char* p = static_cast<volatile char*>(dst);
     for (size_t o = 0; o < bytes; o = (((uintptr_t)dst + o) / page + 1) * page - (uintptr_t)dst) p[o] = p[o];
 }
 
 void download(Context& ctx, void* dst, const void* src, size_t bytes)
 {
-    touch_pages(dst, bytes);
     if (bytes) MNAD_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.d2h += bytes;
 }
