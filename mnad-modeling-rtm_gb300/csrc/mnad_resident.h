@@ -119,6 +119,13 @@ MNAD_HD int res_tasks(int nj, int ni, bool small)
 // Cost of a 4-row group whose points lie in a strip, on top of the plain
 // stencil's 1, per strip direction.
 constexpr double RES_STRIP_COST = 1.0;
+// The same where the patches hold RES_FEW points or fewer on average: a step is
+// then one or two tasks per warp and the exchange, which a wider patch in the
+// interior only lengthens.  201 x 201 2.18 -> 1.94 us a step, 250 x 220 2.38 ->
+// 2.20, 300 x 300 2.69 -> 2.57, 96 x 112 1.69 -> 1.73 (350 x 420, 967 points per
+// patch, 2.89 -> 2.96: not below RES_FEW).
+constexpr double RES_STRIP_COST_FEW = 0.3;
+constexpr int RES_FEW = 640;
 // Fewer groups per CTA than this do not shorten a step, which then costs the
 // exchange of the halo.
 constexpr int RES_MIN_QUADS = 32;
@@ -133,6 +140,7 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
     ResPlan best;
     const double all = (double)nq * nx;
     ncta = std::min(ncta, RES_MAX_PATCHES);
+    const double strip = (double)nz * nx <= (double)RES_FEW * ncta ? RES_STRIP_COST_FEW : RES_STRIP_COST;
     ncta = (int)std::min<double>(ncta, std::max(1.0, std::ceil(all / RES_MIN_QUADS)));
     const int nb0 = (nq + RES_MAX_ROWS / 4 - 1) / (RES_MAX_ROWS / 4);
     for (int nb = nb0; nb <= std::min(nb0 + 4, nq) && nb <= ncta; ++nb) {
@@ -142,13 +150,13 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
         auto colcost = [&](int j0, int nj) {
             ResPatch p{j0, nj, 0, 1};
             const ResLayout L = res_layout(p, nz, nx, d);
-            return nj / 4 + RES_STRIP_COST * (L.zt + L.zb) / 4;
+            return nj / 4 + strip * (L.zt + L.zb) / 4;
         };
         auto cut = [&](double bound, std::vector<ResPatch>* out, std::vector<int>* first) {
             int count = 0;
             for (int b = 0; b < nb; ++b) {
                 const int j0 = row0(b), nj = row0(b + 1) - j0;
-                const double c = colcost(j0, nj), sx = RES_STRIP_COST * (nj / 4);
+                const double c = colcost(j0, nj), sx = strip * (nj / 4);
                 if (first) first->push_back(count);
                 int x = 0;
                 while (x < nx) {
@@ -175,7 +183,7 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
         // bisection between the mean cost of a patch and the best split so far
         double all_cost = 0;
         for (int b = 0; b < nb; ++b)
-            all_cost += colcost(row0(b), row0(b + 1) - row0(b)) * nx + RES_STRIP_COST * (row0(b + 1) - row0(b)) / 4 * strips(nx);
+            all_cost += colcost(row0(b), row0(b + 1) - row0(b)) * nx + strip * (row0(b + 1) - row0(b)) / 4 * strips(nx);
         double lo = all_cost / ncta, hi = best.ok() ? best.cost - 0.5 : all_cost;
         if (hi < lo || cut(hi, nullptr, nullptr) < 0) continue;   // no better, or does not fit at any cost
         for (double m = 2 * lo; !best.ok() && m < hi; m *= 2)
