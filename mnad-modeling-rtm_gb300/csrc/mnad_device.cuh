@@ -148,6 +148,12 @@ struct Coefs2 {
     float2 alpha[NCOEF], beta[NCOEF];
 };
 
+// Device memory to be zeroed: 16-byte aligned, a multiple of 4 bytes.
+struct Span {
+    char* p;
+    unsigned long long bytes;
+};
+
 struct StepArgs {
     Coefs coef;
     Coefs2 coef2;          // TMA kernel

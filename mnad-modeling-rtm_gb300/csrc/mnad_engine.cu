@@ -434,28 +434,37 @@ void Prop::build(Context& ctx)
     }
 }
 
-void Prop::reset(Context& ctx)
+// What a propagation starts from zero.
+std::vector<Span> Prop::zeroed() const
+{
+    std::vector<Span> out;
+    auto add = [&](void* p, size_t bytes) {
+        if (p && bytes) out.push_back(Span{static_cast<char*>(p), bytes});
+    };
+    for (const DevMem* m : {&fields, &mx, &mz, &mx2, &mz2}) add(m->get(), m->size());
+    if (spec.mode == MODE_FWD) {
+        add(data.get(), data.size());
+        add(desc.illum, nint() * sizeof(double));
+        if (spec.wf) add(spec.wf->maxbits.get(), spec.wf->maxbits.size());
+    } else {
+        add(image.get(), image.size());
+    }
+    add(energy.get(), energy.size());
+    return out;
+}
+
+void Prop::reset(Context& ctx, bool zero)
 {
     cudaStream_t st = ctx.stream;
-    MNAD_CK(cudaMemsetAsync(fields.get(), 0, fields.size(), st));
-    for (DevMem* m : {&mx, &mz, &mx2, &mz2})
-        if (m->get()) MNAD_CK(cudaMemsetAsync(m->get(), 0, m->size(), st));
-    if (spec.mode == MODE_FWD) {
-        if (data.get()) MNAD_CK(cudaMemsetAsync(data.get(), 0, data.size(), st));
-        if (desc.illum) MNAD_CK(cudaMemsetAsync(desc.illum, 0, nint() * sizeof(double), st));
-        if (spec.wf && spec.wf->maxbits.get())
-            MNAD_CK(cudaMemsetAsync(spec.wf->maxbits.get(), 0, spec.wf->maxbits.size(), st));
-    } else {
-        if (image.get()) MNAD_CK(cudaMemsetAsync(image.get(), 0, image.size(), st));
-        if (inj.get()) {
-            const size_t n = inj.size() / sizeof(float);
-            const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx.num_sms * 4);
-            // d_desc holds this propagation's data and receiver tables (uploaded at build)
-            injection_table<<<blocks, 256, 0, st>>>(d_desc.as<PropDesc>());
-            MNAD_CK(cudaGetLastError());
-        }
+    if (zero)
+        for (const Span& s : zeroed()) MNAD_CK(cudaMemsetAsync(s.p, 0, s.bytes, st));
+    if (spec.mode == MODE_ADJ && inj.get()) {
+        const size_t n = inj.size() / sizeof(float);
+        const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx.num_sms * 4);
+        // d_desc holds this propagation's data and receiver tables (uploaded at build)
+        injection_table<<<blocks, 256, 0, st>>>(d_desc.as<PropDesc>());
+        MNAD_CK(cudaGetLastError());
     }
-    if (energy.get()) MNAD_CK(cudaMemsetAsync(energy.get(), 0, energy.size(), st));
 }
 
 void Prop::start(Context& ctx, int s_off)
@@ -730,6 +739,21 @@ void Batch::finalize()
         }
     }
     for (Prop* p : props_) upload(ctx_, p->d_desc.get(), &p->desc, sizeof(PropDesc));
+    // what start() zeroes, in pieces of one block each (memsets instead where the
+    // table does not fit the budget)
+    std::vector<Span> spans;
+    for (const Prop* p : props_)
+        for (const Span& s : p->zeroed())
+            for (size_t o = 0; o < s.bytes; o += ZERO_PIECE)
+                spans.push_back(Span{s.p + o, std::min<unsigned long long>(ZERO_PIECE, s.bytes - o)});
+    nspans_ = 0;
+    try {
+        d_spans_ = DevMem(&ctx_, spans.size() * sizeof(Span));
+        upload(ctx_, d_spans_.get(), spans.data(), spans.size() * sizeof(Span));
+        nspans_ = (int)spans.size();
+    } catch (const Error& e) {
+        if (e.code != MNAD_E_BUDGET && e.code != MNAD_E_OOM) throw;
+    }
     d_all_desc_ = DevMem(&ctx_, std::max<size_t>(1, all.size()) * sizeof(PropDesc));
     upload(ctx_, d_all_desc_.get(), all.data(), all.size() * sizeof(PropDesc));
 }
@@ -1010,7 +1034,8 @@ void Batch::launch_group(size_t gi, int s, int slot)
 
 void Batch::start()
 {
-    for (Prop* p : props_) p->reset(ctx_);
+    if (nspans_ > 0) zero_spans<<<nspans_, 256, 0, ctx_.stream>>>(d_spans_.as<Span>());
+    for (Prop* p : props_) p->reset(ctx_, nspans_ == 0);
     if (!props_.empty())
         seed_sources<<<((int)props_.size() + 127) / 128, 128, 0, ctx_.stream>>>(d_all_desc_.as<PropDesc>(),
                                                                             (int)props_.size());
@@ -1247,8 +1272,7 @@ void Batch::run(bool use_graph)
         start();
         launched_ = advance(0, nsteps_);
     };
-    // the state's memsets are most of the launches of an all-resident run; few need no graph
-    if (!use_graph || (all_resident() && props_.size() <= 16)) {
+    if (!use_graph || all_resident()) {        // a few launches need no graph
         body();
         MNAD_CK(cudaGetLastError());
         return;

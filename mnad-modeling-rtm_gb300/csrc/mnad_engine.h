@@ -113,6 +113,7 @@ constexpr double RES_STEP_US = 1.2, RES_QUAD_US = 0.0033;
 // every step 8.0 ms on chip, 4.3 ms step by step; every 4 steps 2.6 and 2.8 ms;
 // every 8 steps 1.7 and 2.6 ms).
 constexpr int RES_MIN_RUN = 6;
+constexpr size_t ZERO_PIECE = 64 << 10;
 constexpr int TUNE_WARMUP = 2, TUNE_STEPS = 8;
 
 // Receivers of one propagation bucketed by TMA_TZ x TMA_TX tile and, within a
@@ -170,7 +171,8 @@ struct Prop {
     DevMem inj;                        // adjoint: injection table [nt][nr] (built by reset())
     const float* r_ext = nullptr;      // set before build(): r shared with other propagations
     void build(Context& ctx);
-    void reset(Context& ctx);          // zero the state of a fresh run; an adjoint also builds
+    std::vector<Span> zeroed() const;
+    void reset(Context& ctx, bool zero = true);          // zero the state of a fresh run; an adjoint also builds
                                        // its injection table from its (final) data (stream-ordered)
     void start(Context& ctx, int s_off);   // reset + seed the source; run from global step s_off (even)
     Checkpoints ckpt;
@@ -261,6 +263,8 @@ private:
     bool tuned_ = false;
     std::vector<Prop*> props_;
     std::vector<std::unique_ptr<LaunchGroup>> groups_;
+    DevMem d_spans_;                   // what start() zeroes, ZERO_PIECE bytes at most each
+    int nspans_ = 0;
     DevMem d_all_desc_;                // every descriptor (source seeding)
     DevMem d_counters_;                // per step and group: tiles claimed (TMA kernel)
     int ntiles_ = 0, nsteps_ = 0;

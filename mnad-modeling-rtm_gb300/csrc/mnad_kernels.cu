@@ -94,6 +94,17 @@ __global__ void injection_table(const PropDesc* __restrict__ desc)
     }
 }
 
+// The state of all propagations of a batch in one launch: five or six memsets per
+// propagation cost about 2 us each whatever their size (18 propagations of
+// 256 x 256: 0.2 ms of a pass of 8.9).
+__global__ void zero_spans(const Span* __restrict__ spans)
+{
+    const Span s = spans[blockIdx.x];
+    const unsigned n = (unsigned)(s.bytes / 16);
+    for (unsigned k = threadIdx.x; k < n; k += blockDim.x) reinterpret_cast<float4*>(s.p)[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (unsigned k = 16 * n + 4 * threadIdx.x; k < s.bytes; k += 4 * blockDim.x) *reinterpret_cast<float*>(s.p + k) = 0.0f;
+}
+
 // U(zs,xs) of the first step holds r_src*w(1) (the injection of tt=1).
 __global__ void seed_sources(const PropDesc* __restrict__ props, int n)
 {

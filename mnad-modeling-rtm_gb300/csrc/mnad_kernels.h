@@ -55,6 +55,8 @@ __global__ void step_resident_small(const __grid_constant__ ResArgs A);
 __global__ void step_resident_small_point(const __grid_constant__ ResArgs A);
 __global__ void build_r(const double* __restrict__ v, int nz, int nx, double dt, int adjoint,
                         float* __restrict__ r, int ld);
+// Zeroes the spans, one block each.
+__global__ void zero_spans(const Span* __restrict__ spans);
 __global__ void seed_sources(const PropDesc* __restrict__ props, int n);
 __global__ void injection_table(const PropDesc* __restrict__ desc);
 __global__ void snap_export(const void* __restrict__ snap, int codec, const float* __restrict__ scale,
