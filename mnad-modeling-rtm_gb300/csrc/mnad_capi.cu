@@ -155,7 +155,6 @@ MNAD_API int mnad_fwd_pde_exact(mnad_context* ctx, double dx, double xs, const d
         b.finalize();
         b.run(false);              // one run: launching directly overlaps the GPU, a capture does not
         const size_t nd = (size_t)nt * nr;
-        touch_pages(datau, nd * sizeof(double));
         download(c, datau, p.data.get(), nd * sizeof(double));
         if (s.record_vw && datav) download(c, datav, p.datav.get(), nd * sizeof(double));
         if (s.record_vw && dataw) download(c, dataw, p.dataw.get(), nd * sizeof(double));
@@ -217,12 +216,10 @@ MNAD_API int mnad_fwd_fields(mnad_context* ctx, double dx, double xs, const doub
                     p.desc.fld[lvl][f], nz, nx, p.desc.ld, f == 0 ? p.desc.src : -1, f == 0 ? fix : 0.0f,
                     tmp.as<double>());
                 MNAD_CK(cudaGetLastError());
-                touch_pages(fields + ((size_t)k * 3 + f) * N, N * sizeof(double));
                 download(c, fields + ((size_t)k * 3 + f) * N, tmp.get(), N * sizeof(double));
             }
         }
         b.advance(done, nt);
-        touch_pages(datau, (size_t)nt * nr * sizeof(double));
         download(c, datau, p.data.get(), (size_t)nt * nr * sizeof(double));
         c.last_energy.assign(p.energy.size() / sizeof(double), 0.0);
         if (!c.last_energy.empty()) download(c, c.last_energy.data(), p.energy.get(), p.energy.size());
@@ -292,7 +289,6 @@ MNAD_API int mnad_born_adj(mnad_context* ctx, double dx, double dz, int nt, doub
         b.finalize();
         b.run(false);              // one run: launching directly overlaps the GPU, a capture does not
         const size_t n = p.nint();
-        touch_pages(im, n * sizeof(double));
         DevMem out(&c, n * sizeof(double));
         scale_f64<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, c.stream>>>(p.image.as<double>(), (double)T, n,
                                                                                         out.as<double>());

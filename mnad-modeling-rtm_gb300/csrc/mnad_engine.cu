@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 namespace mnad {
@@ -124,16 +125,21 @@ void upload(Context& ctx, void* dst, const void* src, size_t bytes)
     ctx.h2d += bytes;
 }
 
-void touch_pages(void* dst, size_t bytes)
+static void populate_pages(void* dst, size_t bytes)
 {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    if (bytes < TOUCH_MIN || bytes > TOUCH_MAX) return;
-    volatile char* p = static_cast<volatile char*>(dst);
-    for (size_t o = 0; o < bytes; o = (((uintptr_t)dst + o) / page + 1) * page - (uintptr_t)dst) p[o] = p[o];
+    if (!dst || bytes < POPULATE_MIN || bytes > POPULATE_MAX) return;
+    const uintptr_t a = (uintptr_t)dst / page * page, b = ((uintptr_t)dst + bytes + page - 1) / page * page;
+#ifdef MADV_POPULATE_WRITE
+    madvise((void*)a, b - a, MADV_POPULATE_WRITE);
+#else
+    (void)a, (void)b;
+#endif
 }
 
 void download(Context& ctx, void* dst, const void* src, size_t bytes)
 {
+    populate_pages(dst, bytes);
     if (bytes) MNAD_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.d2h += bytes;
 }

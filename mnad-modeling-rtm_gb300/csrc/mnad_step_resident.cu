@@ -24,7 +24,7 @@
 // about equal weight; with a few hundred points the exchange, about 1 us from
 // a published cell to its use.  Time per step of one propagation, on chip /
 // the step-per-launch kernel it replaces (CUDA events, GB300):
-//   96 x 112 1.7 / 4.1 us, 201 x 201 2.1 / 4.6, 381 x 681 3.3 / 8.7,
+//   96 x 112 1.7 / 4.1 us, 201 x 201 1.95 / 4.6, 381 x 681 3.3 / 8.7,
 //   481 x 1281 5.1 / 16.9, 600 x 1200 (persistent kernel's rounding) 5.2 / 11.4,
 //   eight of 256 x 256 0.65 / 1.74 each, eight of 321 x 641 2.0 / 3.3 each.
 // Layouts that measured worse on 481 x 1281: one lane group per column with
