@@ -105,6 +105,12 @@ def test_rtm_of_large_patches_and_of_the_persistent_rounding():
     same([shot(420, 820, 20, 60, zs=200, xs=410, seed=k) for k in range(2)], "rtm", T=5, codec="bf16")
 
 
+@pytest.mark.parametrize("receivers", ["field", "deep"])
+def test_receivers_of_large_patches(receivers):
+    """More receivers in a patch than its own table holds; several at one point."""
+    same([shot(250, 500, 20, 70, receivers=receivers, zs=12, xs=14)], "rtm", T=3, codec="bf16")
+
+
 @pytest.mark.parametrize("nt", [1, 2, 3])
 def test_shortest_records(nt):
     same([shot(90, 60, 8, nt)], "rtm", T=1)
