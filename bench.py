@@ -390,6 +390,10 @@ def run_ours(args):
             "kernel": "mnad::step_" + (kernels["forward"] or "tma"),
             "kernels_by_phase": kernels,
             "algorithmic_bytes_per_launch": abytes / plan.timing()["step_launches"]}
+    if "resident" in kernels.values():
+        # the on-chip kernel keeps the state in shared memory: the rate is that of
+        # the bytes a step-per-launch kernel would have to move
+        roof.update(bound="on-chip", traffic=None, note="equivalent HBM rate; the state stays in shared memory")
     # the same roofline split by phase (forwards with snapshots; adjoints with imaging)
     ph = plan.phases()
     roof["phases"] = {

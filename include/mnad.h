@@ -105,7 +105,8 @@ typedef struct mnad_options {
                              (SRC/MNAD/fwd_PDE_exact_MNAD.m:46-47) */
     int record_vw;        /* forward also records V and W (reference keeps
                              them commented out, fwd_PDE_exact_MNAD.m:167-168) */
-    int use_graphs;       /* capture the time loop in a CUDA graph (default 1) */
+    int use_graphs;       /* capture a plan's time loop in a CUDA graph (default 1;
+                             calls that run once launch it directly) */
     int kernel;           /* MNAD_KERNEL_*; default AUTO */
     int energy_every;     /* > 0: FP64 energy diagnostic of each forward every
                              that many steps (read with mnad_context_energy) */
