@@ -1030,11 +1030,11 @@ void Batch::launch_group(size_t gi, int s, int slot)
             cfg.blockDim = dim3(TMA_TZY * TMA_TX_NARROW);
             cfg.dynamicSmemBytes = step_tma_narrow_smem_bytes();
             MNAD_CK(cudaLaunchKernelEx(&cfg, step_tma_narrow, a));
-        }
-        else if (g->kind == MNAD_KERNEL_TMA2)
+        } else if (g->kind == MNAD_KERNEL_TMA2) {
             step_tma2<<<grid, TMA_THREADS, step_tma2_smem_bytes(), ctx_.stream>>>(a);
-        else
+        } else {
             step_direct<<<g->ntiles, dim3(DIRECT_TZ, DIRECT_TX), 0, ctx_.stream>>>(a);
+        }
     }
 }
 
