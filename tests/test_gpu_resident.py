@@ -122,6 +122,28 @@ def test_batches_share_launches():
     same([shot(260, 520, 20, 50 + k, seed=k) for k in range(9)], "model")
 
 
+# byte counts off 16 and off the pieces that are zeroed at a time; every buffer
+# a run adds to (records, images, illumination, FP16 maxima)
+@pytest.mark.parametrize("kernel", ["auto", "direct", "tma"])
+@pytest.mark.parametrize("nz,nx,d,nt,codec", [(41, 37, 4, 33, "f32"), (151, 111, 13, 51, "f16"), (300, 257, 20, 40, "bf16")])
+def test_a_run_leaves_nothing_to_the_next(kernel, nz, nx, d, nt, codec):
+    s = shot(nz, nx, d, nt)
+    out = []
+    for runs in (1, 3):
+        j = mnad.ShotJob("rtm", s["v"], s["dx"], s["dz"], s["dt"], s["nt"], s["d"], s["zs"], s["xs"], s["zr"], s["xr"],
+                         s["w"], vs=s["vs"], T=2)
+        with mnad.Context(0, kernel=kernel, snapshot_codec=codec) as ctx:
+            p = ctx.plan([j])
+            for _ in range(runs):
+                p.run()
+            p.download()
+            p.close()
+        out.append([j.data, j.image, j.illum])
+    assert np.abs(out[0][1]).max() > 0
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
 def test_a_plan_of_resident_and_other_groups():
     """Both in one captured run; launches counted as issued."""
     shots = [shot(90, 90, 8, 40), shot(1000, 1300, 8, 40)]
