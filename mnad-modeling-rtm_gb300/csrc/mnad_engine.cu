@@ -939,7 +939,7 @@ bool Batch::setup_resident(LaunchGroup& g)
         g.wave = w.second;
         g.point_order = g.kind == MNAD_KERNEL_DIRECT;
         g.kind = MNAD_KERNEL_RESIDENT;
-        MNAD_CK(cudaFuncSetAttribute(resident_kernel(g), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM_LIMIT - 1024));
+        MNAD_CK(cudaFuncSetAttribute(resident_kernel(g), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM_LIMIT));
         g.tiles_per_prop = np;
         g.ntiles = np * n;
         return true;

@@ -28,7 +28,10 @@ constexpr int RES_SMALL = 1024;         // points of a patch that goes point by 
 constexpr int RES_MAX_PATCHES = 256;    // CTAs of a propagation at most
 // a plan on the device, in 16-byte units: the patches, then the bands' first patches
 constexpr int RES_TABLE = RES_MAX_PATCHES + (RES_MAX_PATCHES + 1 + 3) / 4;
-constexpr size_t RES_SMEM_LIMIT = 227 * 1024;
+// Shared memory of a CTA: what the device gives, less the kernel's own static
+// part (the descriptor and the patch).
+constexpr size_t RES_SMEM_STATIC = 1024;
+constexpr size_t RES_SMEM_LIMIT = 227 * 1024 - RES_SMEM_STATIC;
 
 // Rows j0 .. j0+nj-1 (a multiple of 4, rows past nz are zero) and columns
 // i0 .. i0+ni-1 of the grid.
@@ -105,7 +108,7 @@ struct ResPlan {
     int slots = 0, threads = 0, comm = 0;  // comm: threads that do the exchange
     bool small = true;                  // all patches go point by point
     double cost = 0;                    // of the costliest patch, in plain quads
-    bool ok() const { return !patches.empty(); }
+    bool ok() const { return !patches.empty() && smem <= RES_SMEM_LIMIT; }
 };
 
 // A step of a patch is a list of warp tasks.  If all patches of a plan are
@@ -165,7 +168,7 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
                     auto fits = [&](int e) {
                         const ResPatch p{j0, nj, x, e - x};
                         return c * e + sx * strips(e) - base <= bound &&
-                               (size_t)res_layout(p, nz, nx, d).total * 4 <= RES_SMEM_LIMIT - 1024;
+                               (size_t)res_layout(p, nz, nx, d).total * 4 <= RES_SMEM_LIMIT;
                     };
                     if (!fits(lo)) return -1;
                     while (lo < hi) {
@@ -197,7 +200,9 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
         p.cost = hi;
         for (const ResPatch& q : p.patches) {
             p.slots = std::max(p.slots, res_slots(q.nj, q.ni));
-            p.small &= q.nj * q.ni <= RES_SMALL;
+            // a table entry per point takes 48 bytes more per group than the
+            // layout that the cut above was held to
+            p.small &= q.nj * q.ni <= RES_SMALL && (size_t)res_layout(q, nz, nx, d, true).total * 4 <= RES_SMEM_LIMIT;
         }
         int tasks = 0;
         for (const ResPatch& q : p.patches) {

@@ -833,6 +833,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(16) PropDesc P;
     __shared__ PatchCtx C;
+    static_assert(sizeof(PropDesc) + sizeof(PatchCtx) + 16 <= RES_SMEM_STATIC, "the dynamic part leaves no room for these");
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int pi = blockIdx.x / A.npatch, me = blockIdx.x - pi * A.npatch;
     {
