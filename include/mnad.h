@@ -64,7 +64,9 @@ enum { MNAD_PAIR_REFERENCE = 0, MNAD_PAIR_ALIGNED = 1 };
 
 /* Step kernel choice.  AUTO picks per launch group (propagations of one grid
  * size advancing together).  Where the state of one propagation fits the SMs'
- * shared memory (up to about 0.7M points) it is RESIDENT: the on-chip kernel,
+ * shared memory (up to about 0.7M points) and an estimate of both sides does
+ * not speak against it (few steps between two returns to the host, large batches
+ * of some grids), it is RESIDENT: the on-chip kernel,
  * which runs all steps of a propagation in one launch; its outputs are bitwise
  * those of the kernel AUTO would take without it.  RESIDENT is reported by
  * mnad_plan_kernels and cannot be set.  Otherwise: the persistent TMA kernel

@@ -896,8 +896,9 @@ static auto resident_kernel(const LaunchGroup& g)
 }
 
 // The on-chip kernel for a group that the AUTO rule has given g.kind: false
-// where a propagation's state does not fit the SMs, or the device memory for
-// the published cells is not to be had (the group then runs g.kind).
+// where a propagation's state does not fit the SMs, where g.kind is expected to
+// be faster (res_pays), or where the device memory for the published cells is not
+// to be had; the group then runs g.kind.
 bool Batch::setup_resident(LaunchGroup& g)
 {
     const int n = (int)g.props.size(), S = ctx_.num_sms;
@@ -923,6 +924,7 @@ bool Batch::setup_resident(LaunchGroup& g)
             continue;
         }
         const int np = (int)p.patches.size();
+        if (!resident_pays(g, p, w.second)) return false;
         try {
             // the split, the snapshots' maxima, the published cells
             g.res_mem = DevMem(&ctx_, (RES_TABLE + (size_t)w.second * np * 2 * (1 + (np > 1 ? p.slots : 0))) * sizeof(uint4));
@@ -945,6 +947,22 @@ bool Batch::setup_resident(LaunchGroup& g)
         return true;
     }
     return false;
+}
+
+bool Batch::resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) const
+{
+    const int longest = g.props[0]->spec.nt, run = std::min(shortest_run(), longest);
+    // a few steps in one launch: nothing to weigh, either way some 20 us
+    if (g.kind == MNAD_KERNEL_DIRECT && wave >= (int)g.props.size() && run == longest) return true;
+    std::vector<ResRun> runs;
+    for (const Prop* q : g.props) {
+        const PropSpec& sp = q->spec;
+        const int steps = std::min(sp.nt, run);
+        const bool snaps = sp.mode == MODE_FWD && sp.wf && sp.T > 0;
+        runs.push_back(ResRun{steps, snaps ? steps / sp.T : 0, snaps && sp.wf->codec == MNAD_SNAP_F16});
+    }
+    const int tile = g.kind == MNAD_KERNEL_DIRECT ? 0 : g.kind == MNAD_KERNEL_TMA_NARROW ? TMA_TX_NARROW : TMA_TX;
+    return res_pays(p, wave, ctx_.num_sms, g.nz, g.nx, g.d, tile, runs);
 }
 
 int Batch::launch_resident(LaunchGroup& g, int s0, int s1)

@@ -87,7 +87,8 @@ struct Context {
 
 // Step-kernel choice of a batch: MNAD_KERNEL_DIRECT, MNAD_KERNEL_TMA,
 // MNAD_KERNEL_AUTO (per launch group: the on-chip kernel where the state of a
-// propagation fits the SMs; else the TMA kernel once a launch has
+// propagation fits the SMs and is expected to be faster there; else the TMA
+// kernel once a launch has
 // AUTO_TMA_TILES_PER_CTA of its tiles for each resident CTA, the direct
 // kernel below) or MNAD_KERNEL_TUNE (per launch group, measured on the
 // batch's own propagations at its first run; Batch::tune).
@@ -248,6 +249,7 @@ private:
     void launch_group(size_t gi, int s, int slot);
     int launch_resident(LaunchGroup& g, int s0, int s1);
     bool setup_resident(LaunchGroup& g);
+    bool resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) const;
     bool hook_due(int s) const;        // per-step host work follows step s
     bool all_resident() const;         // every group runs the on-chip kernel
     int pick_kind(const LaunchGroup& g) const;

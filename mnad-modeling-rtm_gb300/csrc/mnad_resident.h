@@ -220,4 +220,66 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
     return best;
 }
 
+// ---- on chip or a kernel launched once per step ------------------------------
+// One propagation of a launch group over the steps between two returns to the
+// host: its steps and the snapshots it takes in them.
+struct ResRun {
+    int steps, snaps;
+    bool f16;
+};
+
+// Linear fits of measured times (us, GB300), each over the ranges named; the
+// terms are what a launch or a step has to do.
+//
+// On chip, 293 groups of 0.75 to 12 M points (33 x 2000 to 2000 x 100, strips of
+// 0 to 40 points): a launch loads the state, builds its tables and stores the
+// state (29 to 56 us; standard error of the fit 9 %); a step costs the exchange
+// and the groups of the costliest patch (9 %).
+inline double res_fixed_us(const ResPlan& p, int wave, int sms)
+{
+    return 10.5 + 0.154 * p.smem / 1000.0 * (double)p.patches.size() * wave / sms;
+}
+inline double res_step_us(const ResPlan& p) { return 1.44 + 0.003 * p.cost; }
+// A step of the persistent kernels (same groups, 11 %): the launch, the
+// bytes of the tiles with their z halo, the strips along z and along x.  Of the
+// one-thread-per-point kernel: 96 x 112 to 768 x 768.
+constexpr double TMA_LAUNCH_US = 4.8, DIRECT_LAUNCH_US = 3.8;
+inline double step_prop_us(int nz, int nx, int d, int tile_cols)
+{
+    const double m = 1e-6, z = 2.0 * d * nx, x = 2.0 * d * nz;
+    if (tile_cols == 0) return m * (20.0 * nz * nx + 8.0 * (z + x));
+    return m * (6.6 * ((nz + 63) / 64 * 64 + 22) * (double)((nx + tile_cols - 1) / tile_cols * tile_cols) + 10.5 * x + 18.8 * z);
+}
+
+// Whether the on-chip kernel is expected to run the group's propagations (the
+// longest first, `wave` of them to a launch) faster than the persistent kernel on
+// tiles of `tile_cols` columns (0: the one-thread-per-point kernel).  A state that
+// is loaded and stored for a few steps only, or many propagations that each fill
+// the SMs, are where it is not (time on chip / without):
+//   600 x 1100 d 20, 16 propagations: 8 steps 1.64, 36 steps 1.04, 104 steps 0.90;
+//   128 x 128 d 20, 256: 8 steps 1.54, 24 steps 1.05, 100 steps 0.85;
+//   2000 x 100 d 40, 60: 104 steps 1.20, a step alone 1.11;
+//   481 x 1281 d 40, 19: 104 steps 0.76; 2: 6 steps 1.02, 8 steps 0.9.
+// FP16 snapshots at every step (600 x 1100 d 20, 32 forwards) 1.17, every fourth 1.03.
+// The 5 % are held against the fits' error: of those 293 groups 4 run slower than
+// without the on-chip kernel at 104 steps (by 8 % at most, 512 x 512 d 40), 29 without
+// this rule (by 21 % at most); at 400 steps 1 (by 2 %).
+inline bool res_pays(const ResPlan& p, int wave, int sms, int nz, int nx, int d, int tile_cols, const std::vector<ResRun>& runs)
+{
+    double chip = 0, other = 0;
+    const double prop = step_prop_us(nz, nx, d, tile_cols), mpts = 1e-6 * nz * nx;
+    for (size_t k0 = 0; k0 < runs.size(); k0 += wave) {
+        double snaps = 0;
+        for (size_t k = k0; k < std::min(runs.size(), k0 + wave); ++k) {
+            const ResRun& r = runs[k];
+            // a snapshot: stored by the step itself; an FP16 one is read again and encoded
+            snaps = std::max(snaps, r.snaps * (r.f16 ? 0.009 : 0.0028) * p.cost);
+            other += r.steps * prop + r.snaps * (r.f16 ? 3.3 + 7.5 * mpts : 3.0 * mpts);
+        }
+        chip += res_fixed_us(p, wave, sms) + runs[k0].steps * res_step_us(p) + snaps;
+    }
+    if (!runs.empty()) other += runs[0].steps * (tile_cols ? TMA_LAUNCH_US : DIRECT_LAUNCH_US);
+    return chip <= 0.95 * other;
+}
+
 }  // namespace mnad
