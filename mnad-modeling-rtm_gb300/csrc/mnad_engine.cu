@@ -952,15 +952,22 @@ bool Batch::setup_resident(LaunchGroup& g)
 bool Batch::resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) const
 {
     const int longest = g.props[0]->spec.nt, run = std::min(shortest_run(), longest);
-    // a few steps in one launch: nothing to weigh, either way some 20 us
-    if (g.kind == MNAD_KERNEL_DIRECT && wave >= (int)g.props.size() && run == longest) return true;
     std::vector<ResRun> runs;
+    const PropSpec* counted = nullptr;                // the shots of a survey often share their receivers
+    bool lookups = false, any = false;
     for (const Prop* q : g.props) {
         const PropSpec& sp = q->spec;
+        if (!counted || counted->zr != sp.zr || counted->xr != sp.xr)
+            lookups = sp.zr.size() > (size_t)RES_RECS && res_most_receivers(p, sp.zr, sp.xr) > RES_RECS;
+        counted = &sp;
+        any |= lookups;
         const int steps = std::min(sp.nt, run);
         const bool snaps = sp.mode == MODE_FWD && sp.wf && sp.T > 0;
-        runs.push_back(ResRun{steps, snaps ? steps / sp.T : 0, snaps && sp.wf->codec == MNAD_SNAP_F16});
+        runs.push_back(ResRun{steps, snaps ? steps / sp.T : 0, snaps && sp.wf->codec == MNAD_SNAP_F16,
+                              lookups ? res_scan_us((int)sp.zr.size(), p.comm, sp.mode == MODE_FWD) : 0.0});
     }
+    // a few steps in one launch: nothing to weigh, either way some 20 us
+    if (g.kind == MNAD_KERNEL_DIRECT && wave >= (int)g.props.size() && run == longest && !any) return true;
     const int tile = g.kind == MNAD_KERNEL_DIRECT ? 0 : g.kind == MNAD_KERNEL_TMA_NARROW ? TMA_TX_NARROW : TMA_TX;
     return res_pays(p, wave, ctx_.num_sms, g.nz, g.nx, g.d, tile, runs);
 }

@@ -222,10 +222,12 @@ inline ResPlan res_plan(int nz, int nx, int d, int ncta)
 
 // ---- on chip or a kernel launched once per step ------------------------------
 // One propagation of a launch group over the steps between two returns to the
-// host: its steps and the snapshots it takes in them.
+// host: its steps, the snapshots it takes in them, and what looking up its
+// receivers adds to a step of the on-chip kernel (res_scan_us).
 struct ResRun {
     int steps, snaps;
     bool f16;
+    double scan_us;
 };
 
 // Linear fits of measured times (us, GB300), each over the ranges named; the
@@ -240,6 +242,31 @@ inline double res_fixed_us(const ResPlan& p, int wave, int sms)
     return 10.5 + 0.154 * p.smem / 1000.0 * (double)p.patches.size() * wave / sms;
 }
 inline double res_step_us(const ResPlan& p) { return 1.44 + 0.003 * p.cost; }
+// Receivers of a propagation beyond what a patch's own table holds (RES_RECS) are
+// looked up among all nr of it by that patch's exchange warps at every step: 1024
+// in one patch of 481 x 1281 5.4 -> 15.2 us a step, 4096 48.6; with two such warps
+// (321 x 641) 3.4 -> 6.9 and 25.9; the first 1.7 us pass beside the other warps'
+// work.  An adjoint looks them up where it injects: 1024 6.0 -> 9.7 us, 4096 22.9.
+// Without the on-chip kernel they cost next to nothing (201 x 201, all 40,000 points
+// of it: 7.5 instead of 0.34 ms for 60 steps).
+inline double res_scan_us(int nr, int comm, bool forward)
+{
+    return forward ? std::max(0.0, 0.0105 * nr * 32 / comm - 1.7) : 0.0043 * nr;
+}
+// Receivers in the patch that holds the most of them (rows zr, columns xr, from 0).
+inline int res_most_receivers(const ResPlan& p, const std::vector<int>& zr, const std::vector<int>& xr)
+{
+    std::vector<int> held(p.patches.size(), 0);
+    int most = 0;
+    for (size_t k = 0; k < zr.size(); ++k) {
+        size_t b = 0;                                 // the band of the row, then the patch of the column
+        while (b + 2 < p.band_first.size() && p.patches[p.band_first[b + 1]].j0 <= zr[k]) ++b;
+        const auto first = p.patches.begin() + p.band_first[b], last = p.patches.begin() + p.band_first[b + 1];
+        const auto o = std::upper_bound(first, last, xr[k], [](int x, const ResPatch& q) { return x < q.i0; }) - 1;
+        most = std::max(most, ++held[o - p.patches.begin()]);
+    }
+    return most;
+}
 // A step of the persistent kernels (same groups, 11 %): the launch, the
 // bytes of the tiles with their z halo, the strips along z and along x.  Of the
 // one-thread-per-point kernel: 96 x 112 to 768 x 768.
@@ -269,14 +296,15 @@ inline bool res_pays(const ResPlan& p, int wave, int sms, int nz, int nx, int d,
     double chip = 0, other = 0;
     const double prop = step_prop_us(nz, nx, d, tile_cols), mpts = 1e-6 * nz * nx;
     for (size_t k0 = 0; k0 < runs.size(); k0 += wave) {
-        double snaps = 0;
+        double scan = 0, snaps = 0;
         for (size_t k = k0; k < std::min(runs.size(), k0 + wave); ++k) {
             const ResRun& r = runs[k];
+            scan = std::max(scan, r.scan_us);
             // a snapshot: stored by the step itself; an FP16 one is read again and encoded
             snaps = std::max(snaps, r.snaps * (r.f16 ? 0.009 : 0.0028) * p.cost);
             other += r.steps * prop + r.snaps * (r.f16 ? 3.3 + 7.5 * mpts : 3.0 * mpts);
         }
-        chip += res_fixed_us(p, wave, sms) + runs[k0].steps * res_step_us(p) + snaps;
+        chip += res_fixed_us(p, wave, sms) + runs[k0].steps * (res_step_us(p) + scan) + snaps;
     }
     if (!runs.empty()) other += runs[0].steps * (tile_cols ? TMA_LAUNCH_US : DIRECT_LAUNCH_US);
     return chip <= 0.95 * other;

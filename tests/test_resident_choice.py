@@ -26,7 +26,7 @@ extern "C" int pays(int nz, int nx, int d, int n, int wave, int sms, int tile_co
     const ResPlan p = res_plan(nz, nx, d, sms / wave);
     if (!p.ok()) return 2;
     std::vector<ResRun> runs;
-    for (int k = 0; k < n; ++k) runs.push_back(ResRun{steps, k % 2 ? snaps : 0, f16 != 0});
+    for (int k = 0; k < n; ++k) runs.push_back(ResRun{steps, k % 2 ? snaps : 0, f16 != 0, 0.0});
     return res_pays(p, wave, sms, nz, nx, d, tile_cols, runs);
 }
 """
