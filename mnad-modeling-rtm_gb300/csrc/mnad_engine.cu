@@ -30,20 +30,28 @@ DevMem::DevMem(Context* c, size_t bytes) : ctx_(c), n_(bytes)
     p_ = bytes ? c->alloc(bytes) : nullptr;
 }
 
+DevMem DevMem::spare(Context* c, size_t bytes)
+{
+    DevMem m;
+    m.p_ = bytes ? c->alloc_spare(bytes) : nullptr;
+    if (m.p_) m.ctx_ = c, m.n_ = bytes, m.spare_ = true;
+    return m;
+}
+
 DevMem& DevMem::operator=(DevMem&& o) noexcept
 {
     if (this != &o) {
         reset();
-        ctx_ = o.ctx_; p_ = o.p_; n_ = o.n_;
-        o.ctx_ = nullptr; o.p_ = nullptr; o.n_ = 0;
+        ctx_ = o.ctx_; p_ = o.p_; n_ = o.n_; spare_ = o.spare_;
+        o.ctx_ = nullptr; o.p_ = nullptr; o.n_ = 0; o.spare_ = false;
     }
     return *this;
 }
 
 void DevMem::reset()
 {
-    if (p_ && ctx_) ctx_->release(p_, n_);
-    p_ = nullptr; n_ = 0; ctx_ = nullptr;
+    if (p_ && ctx_) ctx_->release(p_, n_, spare_);
+    p_ = nullptr; n_ = 0; ctx_ = nullptr; spare_ = false;
 }
 
 // ---------------------------------------------------------------------------
@@ -83,20 +91,52 @@ Context::~Context()
 
 void* Context::alloc(size_t bytes)
 {
-    if (budget && in_use + bytes > budget)
+    if (budget && in_use - spare + bytes > budget - std::min(budget, held_back))
         throw Error(MNAD_E_BUDGET, "allocation of " + std::to_string(bytes) + " B exceeds the context budget (" +
-                                       std::to_string(in_use) + " of " + std::to_string(budget) + " B in use)");
+                                       std::to_string(in_use - spare) + " of " + std::to_string(budget - std::min(budget, held_back)) +
+                                       " B in use)");
+    while (budget && in_use + bytes > budget && give_back()) {}
     void* p = nullptr;
-    MNAD_CK(cudaMallocAsync(&p, bytes, stream));
+    cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    while (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();            // callers that wait for memory go on: leave no error behind
+        if (!give_back()) break;
+        e = cudaMallocAsync(&p, bytes, stream);
+    }
+    MNAD_CK(e);
     in_use += bytes;
     peak = std::max(peak, in_use);
     return p;
 }
 
-void Context::release(void* p, size_t bytes)
+void* Context::alloc_spare(size_t bytes)
+{
+    if (budget && in_use + bytes > budget) return nullptr;
+    void* p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    MNAD_CK(e);
+    in_use += bytes;
+    spare += bytes;
+    peak = std::max(peak, in_use);
+    return p;
+}
+
+void Context::release(void* p, size_t bytes, bool from_spare)
 {
     cudaFreeAsync(p, stream);
     in_use -= std::min(in_use, bytes);
+    if (from_spare) spare -= std::min(spare, bytes);
+}
+
+bool Context::give_back()
+{
+    for (Batch* b : batches)
+        if (b->give_back()) return true;
+    return false;
 }
 
 void Context::sync() { MNAD_CK(cudaStreamSynchronize(stream)); }
@@ -615,11 +655,48 @@ double Prop::algorithmic_bytes() const
 // ---------------------------------------------------------------------------
 Batch::~Batch()
 {
+    ctx_.batches.erase(std::remove(ctx_.batches.begin(), ctx_.batches.end(), this), ctx_.batches.end());
+    drop_graphs();
+}
+
+void Batch::drop_graphs()
+{
     if (graph_) cudaGraphExecDestroy(graph_);
     if (tick_graph_) cudaGraphExecDestroy(tick_graph_);
+    graph_ = tick_graph_ = nullptr;
+}
+
+bool Batch::give_back()
+{
+    bool held = d_spans_.get() != nullptr;
+    for (const auto& g : groups_) held |= g->res_mem.get() != nullptr;
+    if (!held) return false;
+    d_spans_.reset();
+    nspans_ = 0;
+    for (auto& g : groups_) g->res_mem.reset();
+    spare_ok_ = false;
+    stale_ = true;
+    return true;
 }
 
 void Batch::finalize()
+{
+    do {
+        stale_ = false;
+        drop_graphs();                 // captured with other groups
+        build_groups();
+    } while (stale_);                  // an allocation after the spare ones needed their room
+}
+
+void Batch::prepare(int nsteps)
+{
+    do {
+        if (stale_) finalize();
+        if (has_tma() && nsteps > 0) reserve_counters(nsteps);
+    } while (stale_);
+}
+
+void Batch::build_groups()
 {
     groups_.clear();
     nsteps_ = 0;
@@ -752,14 +829,10 @@ void Batch::finalize()
         for (const Span& s : p->zeroed())
             for (size_t o = 0; o < s.bytes; o += ZERO_PIECE)
                 spans.push_back(Span{s.p + o, std::min<unsigned long long>(ZERO_PIECE, s.bytes - o)});
-    nspans_ = 0;
-    try {
-        d_spans_ = DevMem(&ctx_, spans.size() * sizeof(Span));
-        upload(ctx_, d_spans_.get(), spans.data(), spans.size() * sizeof(Span));
-        nspans_ = (int)spans.size();
-    } catch (const Error& e) {
-        if (e.code != MNAD_E_BUDGET && e.code != MNAD_E_OOM) throw;
-    }
+    d_spans_.reset();
+    if (spare_ok_) d_spans_ = DevMem::spare(&ctx_, spans.size() * sizeof(Span));
+    nspans_ = d_spans_.get() ? (int)spans.size() : 0;
+    if (nspans_ > 0) upload(ctx_, d_spans_.get(), spans.data(), spans.size() * sizeof(Span));
     d_all_desc_ = DevMem(&ctx_, std::max<size_t>(1, all.size()) * sizeof(PropDesc));
     upload(ctx_, d_all_desc_.get(), all.data(), all.size() * sizeof(PropDesc));
 }
@@ -902,7 +975,7 @@ static auto resident_kernel(const LaunchGroup& g)
 bool Batch::setup_resident(LaunchGroup& g)
 {
     const int n = (int)g.props.size(), S = ctx_.num_sms;
-    if (n == 0 || shortest_run() < RES_MIN_RUN) return false;
+    if (n == 0 || !spare_ok_ || shortest_run() < RES_MIN_RUN) return false;
     // Propagations of like lengths share launches (a launch runs as long as its
     // longest).  How many: the split with the shortest estimated run.
     std::stable_sort(g.props.begin(), g.props.end(), [](const Prop* a, const Prop* b) { return a->spec.nt > b->spec.nt; });
@@ -925,13 +998,9 @@ bool Batch::setup_resident(LaunchGroup& g)
         }
         const int np = (int)p.patches.size();
         if (!resident_pays(g, p, w.second)) return false;
-        try {
-            // the split, the snapshots' maxima, the published cells
-            g.res_mem = DevMem(&ctx_, (RES_TABLE + (size_t)w.second * np * 2 * (1 + (np > 1 ? p.slots : 0))) * sizeof(uint4));
-        } catch (const Error& e) {
-            if (e.code == MNAD_E_BUDGET || e.code == MNAD_E_OOM) return false;
-            throw;
-        }
+        // the split, the snapshots' maxima, the published cells
+        g.res_mem = DevMem::spare(&ctx_, (RES_TABLE + (size_t)w.second * np * 2 * (1 + (np > 1 ? p.slots : 0))) * sizeof(uint4));
+        if (!g.res_mem.get()) return false;
         static_assert(sizeof(ResPatch) == sizeof(int4), "patches travel as int4");
         std::vector<int> table(4 * RES_TABLE, 0);
         std::memcpy(table.data(), p.patches.data(), np * sizeof(ResPatch));
@@ -1065,6 +1134,7 @@ void Batch::launch_group(size_t gi, int s, int slot)
 
 void Batch::start()
 {
+    prepare(0);
     if (nspans_ > 0) zero_spans<<<nspans_, 256, 0, ctx_.stream>>>(d_spans_.as<Span>());
     for (Prop* p : props_) p->reset(ctx_, nspans_ == 0);
     if (!props_.empty())
@@ -1179,6 +1249,7 @@ int Batch::advance(int s0, int s1)
         en |= p->energy.get() != nullptr;
         ck |= p->ckpt.saving && p->ckpt.C > 0;
     }
+    prepare(s1 - s0);
     if (has_tma() && s1 > s0) {
         // one tile counter per step and group, zeroed before these launches
         const size_t need = reserve_counters(s1 - s0);
@@ -1268,6 +1339,7 @@ bool Batch::has_step_hooks() const
 void Batch::tick(int K, bool use_graph)
 {
     if (ntiles_ == 0 || K <= 0) return;
+    prepare(K);                               // allocate outside the capture
     if (!use_graph || has_step_hooks() || all_resident()) {    // a few launches need no graph
         advance(0, K);
         return;
@@ -1275,7 +1347,6 @@ void Batch::tick(int K, bool use_graph)
     if (!tick_graph_ || tick_K_ != K) {
         if (tick_graph_) cudaGraphExecDestroy(tick_graph_);
         tick_graph_ = nullptr;
-        if (has_tma()) reserve_counters(K);   // allocate outside the capture
         cudaGraph_t g = nullptr;
         MNAD_CK(cudaStreamBeginCapture(ctx_.stream, cudaStreamCaptureModeThreadLocal));
         advance(0, K);
@@ -1292,13 +1363,10 @@ void Batch::tick(int K, bool use_graph)
 void Batch::run(bool use_graph)
 {
     if (ntiles_ == 0) return;
-    if (tc_.kind == MNAD_KERNEL_TUNE && !tuned_) {
-        tune();
-        if (graph_) {                      // captured with the kernels of the rule
-            cudaGraphExecDestroy(graph_);
-            graph_ = nullptr;
-        }
-    }
+    if (tc_.kind == MNAD_KERNEL_TUNE && !tuned_) tune();
+    // allocate outside the capture: a graph that allocates memory cannot be
+    // relaunched while that memory is held
+    prepare(nsteps_);
     auto body = [&] {
         start();
         launched_ = advance(0, nsteps_);
@@ -1309,9 +1377,6 @@ void Batch::run(bool use_graph)
         return;
     }
     if (!graph_) {
-        // allocate outside the capture: a graph that allocates memory cannot
-        // be relaunched while that memory is held
-        if (has_tma()) reserve_counters(nsteps_);
         cudaGraph_t g = nullptr;
         MNAD_CK(cudaStreamBeginCapture(ctx_.stream, cudaStreamCaptureModeThreadLocal));
         body();

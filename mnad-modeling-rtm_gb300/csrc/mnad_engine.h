@@ -33,6 +33,8 @@ class DevMem {
 public:
     DevMem() = default;
     DevMem(Context* c, size_t bytes);
+    // Memory that its batch can do without: empty where there is no room for it.
+    static DevMem spare(Context* c, size_t bytes);
     ~DevMem() { reset(); }
     DevMem(DevMem&& o) noexcept { *this = std::move(o); }
     DevMem& operator=(DevMem&& o) noexcept;
@@ -46,6 +48,7 @@ private:
     Context* ctx_ = nullptr;
     void* p_ = nullptr;
     size_t n_ = 0;
+    bool spare_ = false;
 };
 
 // Source-side snapshots + illumination of one shot (the reference's
@@ -58,6 +61,8 @@ struct Wavefield {
     DevMem stage, maxbits;   // FP16 codec: FP32 staging snapshot, per-snapshot max |d2u|
 };
 
+class Batch;
+
 struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -65,6 +70,12 @@ struct Context {
     size_t budget = 0;        // 0: unbounded
     size_t in_use = 0;
     size_t peak = 0;           // largest in_use since creation
+    size_t held_back = 0;      // part of the budget that ordinary allocations leave free (the server's batch tables)
+    // Part of in_use that the batches can do without (the on-chip kernel's exchange
+    // buffers, the table of what start() zeroes): taken only where there is room, and
+    // given back when an allocation needs the room, so that no call is refused for it.
+    size_t spare = 0;
+    std::vector<Batch*> batches;
     uint64_t h2d = 0, d2h = 0;   // bytes copied host->device / device->host
     int num_sms = 0;
     unsigned* d_status = nullptr;    // launch-wide status word, and every propagation's unless it has its own
@@ -80,7 +91,9 @@ struct Context {
     explicit Context(int dev, size_t budget_bytes);
     ~Context();
     void* alloc(size_t bytes);
-    void release(void* p, size_t bytes);
+    void* alloc_spare(size_t bytes);   // null where there is no room
+    void release(void* p, size_t bytes, bool from_spare);
+    bool give_back();                  // one batch's spare memory; false if there is none
     void sync();
     unsigned take_status();
 };
@@ -212,10 +225,19 @@ struct LaunchGroup {
 // step 0, advance without step windows and were built with depth2 storage.
 class Batch {
 public:
-    Batch(Context& ctx, const TileCfg& tc, bool depth2_ok = false) : ctx_(ctx), tc_(tc), depth2_ok_(depth2_ok) {}
+    Batch(Context& ctx, const TileCfg& tc, bool depth2_ok = false) : ctx_(ctx), tc_(tc), depth2_ok_(depth2_ok)
+    {
+        ctx_.batches.push_back(this);
+    }
     ~Batch();
+    Batch(const Batch&) = delete;
+    Batch& operator=(const Batch&) = delete;
     void add(Prop* p) { props_.push_back(p); }
     void finalize();
+    // Frees the batch's spare memory (false if it holds none).  Its groups are built
+    // again, without, before the next step: the launches and the fields on the
+    // device are those of the other kernels, and the outputs stay the same bits.
+    bool give_back();
     void run(bool use_graph);          // start() + every step, optionally as one CUDA graph (async)
     // MNAD_KERNEL_TUNE: time TUNE_STEPS steps of every launch group with
     // each step kernel (after TUNE_WARMUP untimed ones) and keep the faster
@@ -243,6 +265,11 @@ public:
     int tiles() const { return ntiles_; }
     const std::vector<Prop*>& props() const { return props_; }
 private:
+    void build_groups();
+    void prepare(int nsteps);          // groups and counters for nsteps steps: all that a step may have to allocate
+    void drop_graphs();
+    bool stale_ = false;               // spare memory was given back: build the groups again
+    bool spare_ok_ = true;
     int launched_ = 0;
     int window_ = INT_MAX;
     int shortest_run() const;

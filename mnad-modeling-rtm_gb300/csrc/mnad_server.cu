@@ -76,7 +76,7 @@ struct mnad_server {
     std::deque<ServerJob*> queue;            // submitted, not admitted (FIFO)
     std::vector<ServerJob*> running;         // owned by the worker thread
     std::unique_ptr<Batch> batch;
-    size_t budget = 0, reserve = 0;          // HBM budget; part kept for batch tables
+    size_t reserve = 0;                      // part of the HBM budget kept for batch tables
     std::atomic<size_t> mem_in_use{0};       // the context's device bytes, for other threads
     std::atomic<size_t> mem_peak{0};         // the context's largest device bytes so far
     bool dirty = true;
@@ -121,7 +121,7 @@ static unsigned take_job_status(Context& c, ServerJob* j)
 bool mnad_server::admit(ServerJob* j)
 {
     Context& c = *ctx;
-    c.budget = budget - reserve;
+    c.held_back = reserve;
     try {
         const mnad_job& J = j->job;
         j->dev_status = DevMem(&c, sizeof(unsigned));
@@ -146,13 +146,13 @@ bool mnad_server::admit(ServerJob* j)
             j->adj->build(c);
             j->points *= 3;
         }
-        c.budget = budget;
+        c.held_back = 0;
         j->fwd_true->start(c, 0);
         if (j->fwd_bg) j->fwd_bg->start(c, 0);
         j->phase = 1;
         return true;
     } catch (const Error& e) {
-        c.budget = budget;
+        c.held_back = 0;
         free_running_state(j);
         if (e.code == MNAD_E_BUDGET || e.code == MNAD_E_OOM) return false;   // wait for memory
         retire(j, e.code, e.what());
@@ -347,7 +347,6 @@ MNAD_API int mnad_server_create(int device, const mnad_server_options* o, mnad_s
             MNAD_CK(cudaMemGetInfo(&fr, &tot));
             budget = fr / 10 * 9;
         }
-        S->budget = budget;
         S->reserve = std::min<size_t>(budget / 8, size_t(64) << 20);
         S->ctx = std::make_unique<Context>(device, budget);
         S->ctx->opt.snapshot_codec = S->opt.snapshot_codec;
