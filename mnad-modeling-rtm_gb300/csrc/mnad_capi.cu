@@ -613,6 +613,7 @@ MNAD_API int mnad_plan_create(mnad_context* ctx, const mnad_job* jobs, int njobs
             for (int k = 0; k < njobs; ++k)
                 if (P->fwd_bg[k]) window = std::min(window, P->ck_C[k]);
             P->recomp->expect_window(window);
+            P->recomp->starts_apart();
             P->phase3->expect_window(window);
             P->recomp->finalize();
         }

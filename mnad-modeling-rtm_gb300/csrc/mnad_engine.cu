@@ -825,7 +825,7 @@ void Batch::build_groups()
     // what start() zeroes, in pieces of one block each (memsets instead where the
     // table does not fit the budget)
     std::vector<Span> spans;
-    for (const Prop* p : props_)
+    for (const Prop* p : whole_ ? props_ : std::vector<Prop*>())
         for (const Span& s : p->zeroed())
             for (size_t o = 0; o < s.bytes; o += ZERO_PIECE)
                 spans.push_back(Span{s.p + o, std::min<unsigned long long>(ZERO_PIECE, s.bytes - o)});

@@ -245,6 +245,7 @@ public:
     // no trace: run() starts from start(), which resets what they touched.
     void tune();
     void expect_window(int k) { window_ = k; }   // advance() and tick() will run about k steps at a time (before finalize)
+    void starts_apart() { whole_ = false; }      // start() is not called: each propagation starts by itself (before finalize)
     void start();                      // zero all state and seed the sources (async)
     int advance(int s0, int s1);       // launch global steps s0..s1-1 (async); step-kernel launches issued
     void refresh_descs();              // re-upload the descriptors after host-side changes
@@ -270,6 +271,7 @@ private:
     void drop_graphs();
     bool stale_ = false;               // spare memory was given back: build the groups again
     bool spare_ok_ = true;
+    bool whole_ = true;
     int launched_ = 0;
     int window_ = INT_MAX;
     int shortest_run() const;

@@ -290,6 +290,7 @@ void mnad_server::loop()
                     if (j->fwd_bg) batch->add(j->fwd_bg.get());
                 }
                 batch->expect_window(K);
+                batch->starts_apart();
                 batch->finalize();
                 dirty = false;
             }
