@@ -352,7 +352,8 @@ MNAD_API int mnad_server_create(int device, const mnad_server_options* o, mnad_s
         S->ctx = std::make_unique<Context>(device, budget);
         S->ctx->opt.snapshot_codec = S->opt.snapshot_codec;
         S->ctx->opt.kernel = S->opt.kernel;
-        S->tc = tile_cfg(S->opt.kernel);
+        // trial steps cannot run on live propagations: the rule
+        S->tc = tile_cfg(S->opt.kernel == MNAD_KERNEL_TUNE ? MNAD_KERNEL_AUTO : S->opt.kernel);
         mnad_server* raw = S.get();
         S->worker = std::thread([raw] {
             try {
