@@ -84,8 +84,10 @@ enum { MNAD_PAIR_REFERENCE = 0, MNAD_PAIR_ALIGNED = 1 };
  * batches (mnad_run_jobs, plans) without checkpointing, FP16 snapshots or the
  * energy diagnostic; elsewhere TMA2 runs as TMA.
  * TUNE measures the candidates -- one thread per point, TMA (64 x 16 tiles),
- * TMA_NARROW (64 x 8 tiles), and TMA2 where it applies -- on each launch
- * group of a plan or job batch at its first run (10 trial steps each, before
+ * TMA_NARROW (64 x 8 tiles), TMA2 where it applies, and the on-chip kernel
+ * where the state fits -- on each launch
+ * group of a plan or job batch at its first run (10 trial steps each, 64 of the
+ * on-chip kernel, before
  * the run starts from zero state) and keeps the fastest; choices are cached in
  * the context per grid, CPML width and propagation count.  The serving loop
  * treats TUNE as AUTO. */

@@ -722,8 +722,9 @@ void Batch::build_groups()
         nsteps_ = std::max(nsteps_, p->spec.nt);
     }
     for (auto& g : groups_) {
-        g->kind = pick_kind(*g);
-        if (tc_.kind == MNAD_KERNEL_AUTO && setup_resident(*g)) {
+        Chip chip;
+        g->kind = pick_kind(*g, chip);
+        if (chip != CHIP_NO && setup_resident(*g, chip == CHIP_MEASURED)) {
             std::vector<PropDesc> descs;
             for (Prop* p : g->props) {
                 p->desc.tile_base = (int)descs.size() * g->tiles_per_prop;
@@ -850,8 +851,9 @@ bool Batch::depth2_allowed(const LaunchGroup& g) const
     return true;
 }
 
-int Batch::pick_kind(const LaunchGroup& g) const
+int Batch::pick_kind(const LaunchGroup& g, Chip& chip) const
 {
+    chip = CHIP_NO;
     const bool d2 = depth2_allowed(g);
     auto valid = [&](int k) { return k == MNAD_KERNEL_TMA2 && !d2 ? MNAD_KERNEL_TMA : k; };
     if (tc_.kind == MNAD_KERNEL_DIRECT || tc_.kind == MNAD_KERNEL_TMA || tc_.kind == MNAD_KERNEL_TMA2 ||
@@ -859,20 +861,30 @@ int Batch::pick_kind(const LaunchGroup& g) const
         return valid(tc_.kind);
     const double tiles = (double)g.props.size() * ((g.nz + TMA_TZ - 1) / TMA_TZ) * ((g.nx + TMA_TX - 1) / TMA_TX);
     const bool persistent = tiles >= AUTO_TMA_TILES_PER_CTA * ctx_.num_sms * TMA_CTAS_PER_SM;
+    chip = CHIP_WEIGH;
     if (tc_.kind == MNAD_KERNEL_TUNE) {
-        if (trial_kind_ >= 0) return valid(trial_kind_);
-        auto it = ctx_.kernel_choice.find(std::make_tuple(g.nz, g.nx, g.d, (int)g.props.size()));
-        if (it != ctx_.kernel_choice.end()) return valid(it->second);
+        if (trial_kind_ >= 0 && trial_kind_ != MNAD_KERNEL_RESIDENT) {
+            chip = CHIP_NO;
+            return valid(trial_kind_);
+        }
+        if (trial_kind_ == MNAD_KERNEL_RESIDENT) chip = CHIP_MEASURED;
+        auto it = trial_kind_ < 0 ? ctx_.kernel_choice.find(std::make_tuple(g.nz, g.nx, g.d, (int)g.props.size()))
+                                  : ctx_.kernel_choice.end();
+        if (it != ctx_.kernel_choice.end()) {
+            chip = it->second.second ? CHIP_MEASURED : CHIP_NO;
+            return valid(it->second.first);
+        }
         // a group that was not measured itself (the step windows of a
         // checkpointed adjoint leave no room for trial steps): the choice
         // measured on the same grid with the nearest propagation count, if
         // both launches are large enough for the persistent kernels
         int best = -1, gap = INT_MAX;
         for (const auto& kv : ctx_.kernel_choice) {
+            if (trial_kind_ >= 0) break;
             const auto& key = kv.first;
             if (std::get<0>(key) != g.nz || std::get<1>(key) != g.nx || std::get<2>(key) != g.d) continue;
             const int dg = std::abs(std::get<3>(key) - (int)g.props.size());
-            if (dg < gap && kv.second != MNAD_KERNEL_DIRECT) best = kv.second, gap = dg;
+            if (dg < gap && kv.second.first != MNAD_KERNEL_DIRECT) best = kv.second.first, gap = dg;
         }
         if (best >= 0 && persistent) return valid(best);
     }
@@ -898,13 +910,15 @@ void Batch::tune()
     const int ng = (int)groups_.size();
     // candidates: one thread per point, the persistent kernel at one and (where
     // the batch allows it) at two steps per pass; the two-step kernel launches
-    // at even steps only, so its K steps are timed in K/2 launches
+    // at even steps only, so its K steps are timed in K/2 launches.  Last the
+    // on-chip kernel, which takes the rounding of the fastest of these, so that
+    // the outputs do not depend on whether it fits.
     bool any_d2 = false;
     for (const auto& g : groups_) any_d2 |= depth2_allowed(*g);
     const int kinds[4] = {MNAD_KERNEL_DIRECT, MNAD_KERNEL_TMA, MNAD_KERNEL_TMA_NARROW, MNAD_KERNEL_TMA2};
     const int nk = any_d2 ? 4 : 3;
-    std::vector<double> ms[4];
-    std::vector<cudaEvent_t> ev((size_t)2 * K * ng, nullptr);
+    std::vector<double> ms[4], chip(ng, -1.0);      // per group: ms of K steps; chip: -1 where it does not fit
+    std::vector<cudaEvent_t> ev((size_t)2 * std::max(K, 3) * ng, nullptr);
     for (auto& e : ev) MNAD_CK(cudaEventCreate(&e));
     try {
         for (int c = 0; c < nk; ++c) {
@@ -933,6 +947,31 @@ void Batch::tune()
                     ms[c][gi] += x;
                 }
         }
+        // the on-chip kernel: a launch of a few steps and one of more give its fixed
+        // time (loading and storing the state) and a step's; what a step costs in runs
+        // of the length to come
+        const int n1 = std::min(K, nsteps_ / 4), n2 = std::min(TUNE_CHIP_STEPS, nsteps_ - 2 * n1);
+        trial_kind_ = MNAD_KERNEL_RESIDENT;
+        finalize();
+        start();
+        for (int gi = 0; gi < ng && n1 >= 2; ++gi) {
+            LaunchGroup& g = *groups_[gi];
+            if (g.kind != MNAD_KERNEL_RESIDENT) continue;
+            cudaEvent_t* e = &ev[(size_t)3 * gi];
+            launch_resident(g, 0, n1);
+            MNAD_CK(cudaEventRecord(e[0], ctx_.stream));
+            launch_resident(g, n1, 2 * n1);
+            MNAD_CK(cudaEventRecord(e[1], ctx_.stream));
+            launch_resident(g, 2 * n1, 2 * n1 + n2);
+            MNAD_CK(cudaEventRecord(e[2], ctx_.stream));
+            MNAD_CK(cudaStreamSynchronize(ctx_.stream));
+            float a = 0, b = 0;
+            MNAD_CK(cudaEventElapsedTime(&a, e[0], e[1]));
+            MNAD_CK(cudaEventElapsedTime(&b, e[1], e[2]));
+            const double step = std::max(0.0, (double)(b - a) / (n2 - n1)), fixed = std::max(0.0, a - n1 * step);
+            const int run = std::min(shortest_run(), g.props[0]->spec.nt);
+            chip[gi] = K * (step + fixed / run);
+        }
     } catch (...) {
         for (auto& e : ev) cudaEventDestroy(e);
         trial_kind_ = -1;
@@ -944,7 +983,8 @@ void Batch::tune()
         int best = 0;
         for (int c = 1; c < nk; ++c)
             if (ms[c][gi] < ms[best][gi]) best = c;
-        ctx_.kernel_choice[std::make_tuple(g.nz, g.nx, g.d, (int)g.props.size())] = kinds[best];
+        const bool on_chip = chip[gi] >= 0 && chip[gi] < ms[best][gi];
+        ctx_.kernel_choice[std::make_tuple(g.nz, g.nx, g.d, (int)g.props.size())] = {kinds[best], on_chip};
     }
     trial_kind_ = -1;
     finalize();
@@ -971,8 +1011,9 @@ static auto resident_kernel(const LaunchGroup& g)
 // The on-chip kernel for a group that the AUTO rule has given g.kind: false
 // where a propagation's state does not fit the SMs, where g.kind is expected to
 // be faster (res_pays), or where the device memory for the published cells is not
-// to be had; the group then runs g.kind.
-bool Batch::setup_resident(LaunchGroup& g)
+// to be had; the group then runs g.kind.  `measured`: a whole run on chip was
+// measured to be faster.
+bool Batch::setup_resident(LaunchGroup& g, bool measured)
 {
     const int n = (int)g.props.size(), S = ctx_.num_sms;
     if (n == 0 || !spare_ok_ || shortest_run() < RES_MIN_RUN) return false;
@@ -997,7 +1038,7 @@ bool Batch::setup_resident(LaunchGroup& g)
             continue;
         }
         const int np = (int)p.patches.size();
-        if (!resident_pays(g, p, w.second)) return false;
+        if (!resident_pays(g, p, w.second, measured)) return false;
         // the split, the snapshots' maxima, the published cells
         g.res_mem = DevMem::spare(&ctx_, (RES_TABLE + (size_t)w.second * np * 2 * (1 + (np > 1 ? p.slots : 0))) * sizeof(uint4));
         if (!g.res_mem.get()) return false;
@@ -1018,7 +1059,7 @@ bool Batch::setup_resident(LaunchGroup& g)
     return false;
 }
 
-bool Batch::resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) const
+bool Batch::resident_pays(const LaunchGroup& g, const ResPlan& p, int wave, bool measured) const
 {
     const int longest = g.props[0]->spec.nt, run = std::min(shortest_run(), longest);
     std::vector<ResRun> runs;
@@ -1035,6 +1076,7 @@ bool Batch::resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) cons
         runs.push_back(ResRun{steps, snaps ? steps / sp.T : 0, snaps && sp.wf->codec == MNAD_SNAP_F16,
                               lookups ? res_scan_us((int)sp.zr.size(), p.comm, sp.mode == MODE_FWD) : 0.0});
     }
+    if (measured && run == longest && !any) return true;
     // a few steps in one launch: nothing to weigh, either way some 20 us
     if (g.kind == MNAD_KERNEL_DIRECT && wave >= (int)g.props.size() && run == longest && !any) return true;
     const int tile = g.kind == MNAD_KERNEL_DIRECT ? 0 : g.kind == MNAD_KERNEL_TMA_NARROW ? TMA_TX_NARROW : TMA_TX;

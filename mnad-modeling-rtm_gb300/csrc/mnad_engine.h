@@ -81,8 +81,9 @@ struct Context {
     unsigned* d_status = nullptr;    // launch-wide status word, and every propagation's unless it has its own
     unsigned wait_limit = 0;         // polls of a bounded barrier wait in the step kernels (0: default)
     std::map<int, std::unique_ptr<Wavefield>> wavefields;
-    // MNAD_KERNEL_TUNE: measured step kernel per (nz, nx, d_pml, propagations per launch)
-    std::map<std::tuple<int, int, int, int>, int> kernel_choice;
+    // MNAD_KERNEL_TUNE: per (nz, nx, d_pml, propagations per launch) the fastest kernel
+    // that launches once per step, and whether the on-chip kernel was faster still
+    std::map<std::tuple<int, int, int, int>, std::pair<int, bool>> kernel_choice;
     // splits of a grid over CTAs for the on-chip kernel, by (nz, nx, d_pml, CTAs); bounded
     std::map<std::tuple<int, int, int, int>, std::shared_ptr<const ResPlan>> res_plans;
     std::shared_ptr<const ResPlan> resident_plan(int nz, int nx, int d, int ncta);
@@ -128,7 +129,7 @@ constexpr double RES_STEP_US = 1.2, RES_QUAD_US = 0.0033;
 // every 8 steps 1.7 and 2.6 ms).
 constexpr int RES_MIN_RUN = 6;
 constexpr size_t ZERO_PIECE = 64 << 10;
-constexpr int TUNE_WARMUP = 2, TUNE_STEPS = 8;
+constexpr int TUNE_WARMUP = 2, TUNE_STEPS = 8, TUNE_CHIP_STEPS = 48;
 
 // Receivers of one propagation bucketed by TMA_TZ x TMA_TX tile and, within a
 // tile, by column (stable counting sort): entries of tile t are
@@ -277,11 +278,12 @@ private:
     int shortest_run() const;
     void launch_group(size_t gi, int s, int slot);
     int launch_resident(LaunchGroup& g, int s0, int s1);
-    bool setup_resident(LaunchGroup& g);
-    bool resident_pays(const LaunchGroup& g, const ResPlan& p, int wave) const;
+    bool setup_resident(LaunchGroup& g, bool measured);
+    bool resident_pays(const LaunchGroup& g, const ResPlan& p, int wave, bool measured) const;
     bool hook_due(int s) const;        // per-step host work follows step s
     bool all_resident() const;         // every group runs the on-chip kernel
-    int pick_kind(const LaunchGroup& g) const;
+    enum Chip { CHIP_NO, CHIP_WEIGH, CHIP_MEASURED };    // the on-chip kernel: not, where it is expected to pay, as measured
+    int pick_kind(const LaunchGroup& g, Chip& chip) const;
     bool depth2_allowed(const LaunchGroup& g) const;
     size_t reserve_counters(int nsteps);   // tile counters for nsteps steps (bytes used)
     void encode_snapshots(int s);      // FP16 codec: encode the snapshots taken at step s
