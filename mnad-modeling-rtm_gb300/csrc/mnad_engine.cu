@@ -1,6 +1,7 @@
 // Host-side engine: device memory, propagation setup, batched time loop.
 #include "mnad_engine.h"
 #include "mnad_kernels.h"
+#include "mnad_pages.h"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -9,9 +10,6 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
-
-#include <sys/mman.h>
-#include <unistd.h>
 
 namespace mnad {
 
@@ -163,18 +161,6 @@ void upload(Context& ctx, void* dst, const void* src, size_t bytes)
 {
     if (bytes) MNAD_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx.stream));
     ctx.h2d += bytes;
-}
-
-static void populate_pages(void* dst, size_t bytes)
-{
-    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    if (!dst || bytes < POPULATE_MIN || bytes > POPULATE_MAX) return;
-    const uintptr_t a = (uintptr_t)dst / page * page, b = ((uintptr_t)dst + bytes + page - 1) / page * page;
-#ifdef MADV_POPULATE_WRITE
-    madvise((void*)a, b - a, MADV_POPULATE_WRITE);
-#else
-    (void)a, (void)b;
-#endif
 }
 
 void download(Context& ctx, void* dst, const void* src, size_t bytes)

@@ -332,15 +332,7 @@ size_t noalloc_scratch_bytes();
 
 // Device copies of the shot records (FP64, nt x nr).
 void upload(Context& ctx, void* dst, const void* src, size_t bytes);
-// Copies a result to the host, after making the buffer's pages present (no byte
-// changes by that; nothing happens where the range is not mapped).  Fresh host
-// memory (an untouched allocation) is otherwise faulted in by the copy from the
-// device: a shot record into a new array took 5.3 ms instead of 1.8 at 4 MB,
-// 17.7 instead of 4.8 at 16 MB, 32.5 instead of 8.3 at 30 MB (touching page by
-// page 2.2, 6.4 and 11.6), the first download of 16 RTM shots of 481 x 1281
-// 57 instead of 8 ms.  Above 32 MB the driver copies with host threads, which
-// fault as fast.
-constexpr size_t POPULATE_MIN = 256 << 10, POPULATE_MAX = 30 << 20;
+// Copies a result to the host, after making the buffer's pages present (mnad_pages.h).
 void download(Context& ctx, void* dst, const void* src, size_t bytes);
 
 }  // namespace mnad
