@@ -156,10 +156,10 @@ MNAD_API int mnad_context_energy(const mnad_context* ctx, double* out, int max, 
  * clears these flags itself at its end and fails with MNAD_E_NUMERIC (1, 2)
  * or MNAD_E_TIMEOUT (4) when one is set; the context stays usable. */
 MNAD_API int mnad_context_status(mnad_context* ctx, unsigned* flags);
-/* Bound of every barrier wait in the persistent step kernel, in polls of the
- * barrier (0: the default, about 4 M polls -- far longer than any tile copy
- * takes).  A wait that runs out makes the launch give up its remaining
- * tiles, and the call then returns MNAD_E_TIMEOUT.  A diagnostic for
+/* Bound of every wait in the step kernels (for a tile copy's barrier, for a
+ * neighbour's cells on chip), in polls (0: the default, about 4 M -- far longer
+ * than either takes).  A wait that runs out makes the launch give up its
+ * remaining work, and the call then returns MNAD_E_TIMEOUT.  A diagnostic for
  * watchdog tests: a limit of a few polls makes the waits run out on purpose.
  * No counterpart in the reference (its MATLAB loop has no device waits). */
 MNAD_API int mnad_context_set_wait_limit(mnad_context* ctx, unsigned polls);

@@ -144,8 +144,8 @@ PropSpec job_spec(const mnad_job& j, int mode, const double* v, Wavefield* wf, i
 void raise_status(unsigned bits, const std::string& what)
 {
     if (bits & ST_TIMEOUT)
-        throw Error(MNAD_E_TIMEOUT, what + ": a bounded device wait for a tile copy ran out; the outputs are "
-                                           "incomplete (the context stays usable)");
+        throw Error(MNAD_E_TIMEOUT, what + ": a bounded device wait (for a tile copy, or for a neighbour's cells on "
+                                           "chip) ran out; the outputs are incomplete (the context stays usable)");
     if (bits & ST_NONFINITE)
         throw Error(MNAD_E_NUMERIC, what + ": a recorded wavefield value is not finite (unstable time step "
                                            "v*dt/dx, or non-finite input)");

@@ -56,7 +56,7 @@ void rtm_snapshot_plan(const mnad_job& j, int& T, int& ncols, ModelScans* scans 
 // Propagation spec of a job: forward (true or background model) or adjoint.
 PropSpec job_spec(const mnad_job& j, int mode, const double* v, Wavefield* wf, int T, int pairing);
 // Device status bits -> error: ST_TIMEOUT throws MNAD_E_TIMEOUT (a step
-// launch gave up on a tile copy, so the outputs are incomplete), ST_NONFINITE
+// launch gave up on a tile copy or on a neighbour's cells, so the outputs are incomplete), ST_NONFINITE
 // or ST_F16_RANGE throw MNAD_E_NUMERIC (a recorded value was not finite or a
 // snapshot saturated).  `what` names the call.
 void raise_status(unsigned bits, const std::string& what);
