@@ -125,6 +125,28 @@ def peaks():
         return 6800.0, "fallback"
 
 
+FLOPS_PER_POINT = 137        # of the stencil and the update, without the CPML strips
+
+
+def fp32_peak(sm_max_mhz):
+    """TFLOP/s of the FP32 pipes: 128 lanes per SM, two operations per lane and cycle."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 152
+    return sms * 128 * 2 * (sm_max_mhz or 2070.0) * 1e6 / 1e12
+
+
+def kernel_roof(kernel, pts, nbytes, seconds, hbm_peak, fp32):
+    """What bounds a step kernel and how near it is: HBM for the kernels that move the
+    state once per step (algorithmic bytes), the FP32 rate for the on-chip kernel, which
+    keeps the state in shared memory."""
+    if kernel == "resident":
+        a = FLOPS_PER_POINT * pts / seconds / 1e12
+        return {"bound": "fp32", "achieved": round(a, 2), "peak": round(fp32, 1), "unit": "TFLOP/s", "frac": round(a / fp32, 4),
+                "peak_kind": "128 lanes x SMs x 2 x max SM clock"}
+    a = nbytes / seconds / 1e9
+    return {"bound": "hbm", "achieved": round(a, 1), "peak": hbm_peak, "unit": "GB/s", "frac": round(a / hbm_peak, 4)}
+
+
 def profile_traffic():
     """DRAM bytes per point-update of the step kernel from the committed ncu summary."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
@@ -379,28 +401,27 @@ def run_ours(args):
     ms_per_step = total_s * 1e3 / args.steps
     shots_hr = allsum(len(jobs) * args.steps, world) / total_s * 3600.0
     peak, peak_kind = peaks()
-    achieved = abytes * args.steps / (sum(step_ms) / 1e3) / 1e9
+    fp32 = fp32_peak(clocks.get("sm_max_mhz"))
     tr = profile_traffic()
     traffic = None
     if tr and "bytes_per_point_update" in tr and args.workload == "random-field":
         traffic = tr["bytes_per_point_update"] * pts / (plan.timing()["step_launches"])
-    roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "traffic": traffic,
-            "peak_kind": f"{peak_kind} hbm_gbs",
+    roof = {"traffic": traffic, "peak_kind": f"{peak_kind} hbm_gbs",
             "kernel": "mnad::step_" + (kernels["forward"] or "tma"),
             "kernels_by_phase": kernels,
-            "algorithmic_bytes_per_launch": abytes / plan.timing()["step_launches"]}
-    if "resident" in kernels.values():
-        # the on-chip kernel keeps the state in shared memory: the rate is that of
-        # the bytes a step-per-launch kernel would have to move
-        roof.update(bound="on-chip", traffic=None, note="equivalent HBM rate; the state stays in shared memory")
+            "algorithmic_bytes_per_launch": abytes / plan.timing()["step_launches"],
+            **kernel_roof(kernels["forward"], pts * args.steps, abytes * args.steps, sum(step_ms) / 1e3, peak, fp32)}
+    if roof["bound"] == "fp32":
+        roof["traffic"] = None
     # the same roofline split by phase (forwards with snapshots; adjoints with imaging)
     ph = plan.phases()
-    roof["phases"] = {
-        name: {"ms_per_step": round(ms / args.steps, 1),
-               "achieved": round(b * args.steps / (ms / 1e3) / 1e9, 1) if ms > 0 else None,
-               "frac": round(b * args.steps / (ms / 1e3) / 1e9 / peak, 4) if ms > 0 else None}
-        for name, ms, b in (("forward", phase_ms[0], ph["forward_bytes"]), ("adjoint", phase_ms[1], ph["adjoint_bytes"]))}
+    roof["phases"] = {}
+    for name, ms in zip(("forward", "adjoint"), phase_ms):
+        b = ph[name + "_bytes"]
+        # its share of the point updates: by algorithmic bytes, which are near 40 per update in both
+        r = kernel_roof(kernels[name], pts * b / abytes * args.steps, b * args.steps, ms / 1e3, peak, fp32) if ms > 0 else {}
+        roof["phases"][name] = {"ms_per_step": round(ms / args.steps, 1), "achieved": r.get("achieved"), "frac": r.get("frac"),
+                                "unit": r.get("unit")}
     # the one exchange of the path: the FP64 image / illumination stack over ranks
     t = time.perf_counter()
     im, il, _ = plan.stack()
