@@ -110,7 +110,8 @@ struct TileCfg {
     int kind;     // MNAD_KERNEL_*
 };
 TileCfg tile_cfg(int kernel);
-// Measured crossover of the two step kernels on GB300 (152 SMs, 2 CTAs per
+// For groups that do not run on chip, and for the rounding of those that do:
+// measured crossover of the two step kernels on GB300 (152 SMs, 2 CTAs per
 // SM; grids of 96^2 to 2048^2, 1 to 8 propagations per launch): the direct
 // kernel wins up to 0.59M point-updates per launch (575 tiles, 1.9 per CTA),
 // the persistent TMA kernel from 0.82M (800 tiles, 2.6 per CTA) on; its

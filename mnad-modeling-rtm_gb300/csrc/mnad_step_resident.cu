@@ -1126,6 +1126,7 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
                 // 600 cycles: 481 x 1281 5.45 -> 5.10 us a step, 381 x 681 3.50
                 // -> 3.30, 600 x 1200 5.69 -> 5.20 (300: 5.20, 3.38, 5.31; 900:
                 // 5.25, 3.21, 5.28; turns passed by named barriers: 5.69, 3.45, 5.74).
+                // All of these plans go round twice or more; one round was not measured.
                 const unsigned t0 = clock(), wait = (tid >> 7) * RES_STAGGER;
                 while ((unsigned)clock() - t0 < wait) {}
             }
@@ -1183,6 +1184,8 @@ __device__ __forceinline__ void resident_body(const ResArgs& A)
                     for (int k = ct; k < C.nrec; k += comm) fill_injection(s + 1, k);
                 const uint4* in = C.words + ((s + 1) & 1) * C.plane;
                 const int nhalo = C.nhalo;
+                // all cells in one round of polls where 3 or 6 per lane do; more per
+                // lane and round than 11 (12, 16, 20) measured the same
                 if (nhalo <= 0) {
                 } else if (nhalo <= 3 * comm) {
                     bad = !collect<3>(in, halo, nhalo, S.nxt, fs, S.tag, ct, comm, A);
